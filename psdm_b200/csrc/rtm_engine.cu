@@ -15,6 +15,7 @@
 #include <array>
 #include <complex>
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -100,6 +101,26 @@ struct psdm_engine {
     std::vector<int> res_key[2];   // resident form, by pass kind
     int res_nreg[2] = {0, 0}, res_sw[2] = {0, 0};
     cudaEvent_t pass_staged[3] = {nullptr, nullptr, nullptr};  // copies out of the staging buffers done
+    // Until a launch form is chosen (psdm_engine_set_pass_launch), passes run
+    // as one region launch each where the grid fits (rtm_region.cu).
+    bool use_regions = true;
+    // Region plans by (ny, nx, dPML, fs, regions), each with its lists in
+    // buffers of its own; the oldest gives way.
+    struct RegSlot {
+        std::array<int, 5> key{};
+        bool used = false, fits = false;
+        RegPlan plan;
+        RegBlock* d_blocks = nullptr;
+        RegPair* d_pub = nullptr;
+        int* d_rcv = nullptr;
+    };
+    static constexpr int kRegPlans = 12;
+    RegSlot reg_plans[kRegPlans];
+    int reg_next = 0;
+    std::map<std::string, cudaEvent_t> reg_staged;  // copies out of a staging buffer done
+    unsigned int reg_epoch = 1;  // tag of the next region launch's first step
+    void* reg_board = nullptr;   // the board whose tags reg_epoch counts
+    size_t reg_board_bytes = 0;
     int batch_slots = 0;  // slots used by the last batched call
     int ckpt_interval = 0;  // > 0: shots keep checkpoints every K steps instead of all snapshots
     std::map<int, cudaGraphExec_t> bgraphs;  // batched launches: an executable graph per run length
@@ -155,6 +176,8 @@ struct psdm_engine {
         drop_graphs();
         for (auto& k : pass_key) k.clear();
         for (auto& k : res_key) k.clear();
+        for (RegSlot& r : reg_plans) r = RegSlot{};
+        reg_board = nullptr;
         for (auto& kv : fft_plans) destroy_fft_plans(kv.second.data());
         fft_plans.clear();
         for (auto& kv : bufs)
@@ -701,6 +724,170 @@ int launch_steps(psdm_engine* e, int mode, const std::vector<StepArgs>& args, in
     return PSDM_OK;
 }
 
+// ---- passes as region launches (rtm_region.cu) --------------------------------
+
+// Cooperative launches of one device follow each other: a block of a region
+// launch waits for its neighbours, so two of them that each hold part of the
+// device would wait for good.  Every region launch of the process waits for
+// the device's previous one, whatever its engine, stream or thread.
+struct CoopOrder {
+    std::mutex m;
+    std::map<int, cudaEvent_t> done;
+};
+CoopOrder& coop_order() {
+    static CoopOrder* o = new CoopOrder;  // outlives every engine
+    return *o;
+}
+
+// The plan of a grid for `regions` blocks, made and uploaded on first use.
+// *out = null if the grid does not fit.
+int region_plan(psdm_engine* e, const Grid& g, int fs, int regions, psdm_engine::RegSlot** out) {
+    const std::array<int, 5> key = {g.ny, g.nx, g.dPML, fs, regions};
+    *out = nullptr;
+    for (auto& r : e->reg_plans)
+        if (r.used && r.key == key) {
+            if (r.fits) *out = &r;
+            return PSDM_OK;
+        }
+    const int k = e->reg_next;
+    auto& r = e->reg_plans[k];
+    e->reg_next = (k + 1) % psdm_engine::kRegPlans;
+    r = psdm_engine::RegSlot{};
+    r.key = key;
+    r.fits = plan_regions(g, fs, regions, region_max_floats(), &r.plan);
+    r.used = true;
+    if (!r.fits) return PSDM_OK;
+    const std::string t = std::to_string(k);
+    r.used = false;  // until the uploads are queued
+    TRY(e->get(("reg_blocks" + t).c_str(), r.plan.blocks.size(), &r.d_blocks));
+    TRY(e->get(("reg_pub" + t).c_str(), std::max<size_t>(r.plan.pub.size(), 1), &r.d_pub));
+    TRY(e->get(("reg_rcv" + t).c_str(), std::max<size_t>(r.plan.rcv.size(), 1), &r.d_rcv));
+    CUDA_TRY(cudaMemcpyAsync(r.d_blocks, r.plan.blocks.data(), r.plan.blocks.size() * sizeof(RegBlock),
+                             cudaMemcpyHostToDevice, e->stream));
+    CUDA_TRY(cudaMemcpyAsync(r.d_pub, r.plan.pub.data(), r.plan.pub.size() * sizeof(RegPair), cudaMemcpyHostToDevice,
+                             e->stream));
+    CUDA_TRY(cudaMemcpyAsync(r.d_rcv, r.plan.rcv.data(), r.plan.rcv.size() * sizeof(int), cudaMemcpyHostToDevice,
+                             e->stream));
+    r.used = true;
+    *out = &r;
+    return PSDM_OK;
+}
+
+// One pass of one shot as region launches: its plan, the device copies of its
+// geometry lists and per-step values.
+struct RegPass {
+    psdm_engine::RegSlot* plan = nullptr;
+    RegParams rp{};
+    size_t floats = 0, floats_img = 0;
+    RegVar* d_var = nullptr;
+    int nsteps = 0;
+};
+
+bool regions_on(const psdm_engine* e) {
+    return e->use_regions && e->use_pass == 0 && e->steps_per_launch == 1 && region_max_floats() > 0;
+}
+
+// Prepare a pass: injection points by last write wins (build_inj's cells),
+// receivers, and the values of its steps.  `kind` names its buffers (passes
+// of different kinds may be queued together).  Returns 1 if the pass does not
+// fit the form.
+int region_prepare(psdm_engine* e, const Shot& s, const InjMap& inj, int nrec, const int* h_rec_cell,
+                   const std::vector<RegVar>& var, const std::string& kind, RegPass* P) {
+    const Grid& g = s.g;
+    TRY(region_plan(e, g, s.fs, e->num_sms, &P->plan));
+    if (!P->plan) return 1;
+    std::vector<int> cell, trace;
+    for (int zd = 0; zd < g.ldz; ++zd) {
+        if (inj.row_slot[zd] < 0) continue;
+        const int* c = inj.cols.data() + (size_t)inj.row_slot[zd] * g.nxt;
+        for (int x = 0; x < g.nxt; ++x)
+            if (c[x] >= 0) {
+                cell.push_back(x * g.ldz + zd);
+                trace.push_back(c[x]);
+            }
+    }
+    RegLists L;
+    if (!region_loads(P->plan->plan, g, region_max_floats(), (int)cell.size(), cell.data(), trace.data(), nrec,
+                      h_rec_cell, &L))
+        return 1;
+    P->floats = L.floats;
+    P->floats_img = L.floats_img;
+    P->nsteps = (int)var.size();
+    // One staging buffer per kind, page-locked, refilled after its last copy.
+    const size_t nb[5] = {var.size() * sizeof(RegVar), L.loads.size() * sizeof(RegLoad),
+                          L.inj.size() * sizeof(RegPair), L.rec.size() * sizeof(RegPair), L.slots.size()};
+    size_t off[6] = {0};
+    for (int k = 0; k < 5; ++k) off[k + 1] = (off[k] + nb[k] + 15) & ~(size_t)15;
+    char *h = nullptr, *d = nullptr;
+    cudaEvent_t& done = e->reg_staged[kind];
+    if (done == nullptr) CUDA_TRY(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
+    CUDA_TRY(cudaEventSynchronize(done));
+    TRY(e->get_pinned(("reg_stage" + kind).c_str(), off[5], reinterpret_cast<void**>(&h)));
+    TRY(e->get(("reg_pass" + kind).c_str(), off[5], &d));
+    const void* src[5] = {var.data(), L.loads.data(), L.inj.data(), L.rec.data(), L.slots.data()};
+    for (int k = 0; k < 5; ++k)
+        if (nb[k]) std::memcpy(h + off[k], src[k], nb[k]);
+    CUDA_TRY(cudaMemcpyAsync(d, h, off[5], cudaMemcpyHostToDevice, e->stream));
+    CUDA_TRY(cudaEventRecord(done, e->stream));
+    P->d_var = reinterpret_cast<RegVar*>(d);
+    RegParams& rp = P->rp;
+    rp.jobs = nullptr;
+    rp.neg0 = -0.0f;
+    rp.blocks = P->plan->d_blocks;
+    rp.pub = P->plan->d_pub;
+    rp.rcv = P->plan->d_rcv;
+    rp.loads = reinterpret_cast<const RegLoad*>(d + off[1]);
+    rp.inj = reinterpret_cast<const RegPair*>(d + off[2]);
+    rp.rec = reinterpret_cast<const RegPair*>(d + off[3]);
+    rp.slots = reinterpret_cast<const signed char*>(d + off[4]);
+    return PSDM_OK;
+}
+
+// The board of `npk` packets a plane and the tag of its next launch of
+// `nsteps` steps; tags never repeat on a board.
+int region_board(psdm_engine* e, size_t npk, int nsteps, void** board, unsigned int* epoch) {
+    const size_t bytes = std::max<size_t>(npk, 1) * 32;
+    char* b = nullptr;
+    TRY(e->get("reg_board", bytes, &b));
+    const size_t have = e->bufs["reg_board"].bytes;
+    if (b != e->reg_board || have != e->reg_board_bytes || e->reg_epoch > 0xffffffffu - (unsigned int)nsteps - 1u) {
+        CUDA_TRY(cudaMemsetAsync(b, 0, have, e->stream));
+        e->reg_board = b;
+        e->reg_board_bytes = have;
+        e->reg_epoch = 1;
+    }
+    *board = b;
+    *epoch = e->reg_epoch;
+    e->reg_epoch += (unsigned int)nsteps;
+    return PSDM_OK;
+}
+
+// Launch steps [i0, i1) of a prepared pass; `a` = the arguments of step i0.
+int region_launch(psdm_engine* e, int mode, RegPass& P, const StepArgs& a, int i0, int i1) {
+    if (i1 <= i0) return PSDM_OK;
+    RegParams& rp = P.rp;
+    rp.job = RegJob{};
+    rp.job.a = a;
+    rp.job.var = P.d_var + i0;
+    rp.job.nsteps = i1 - i0;
+    rp.job.npk = P.plan->plan.npk;
+    TRY(region_board(e, (size_t)rp.job.npk, rp.job.nsteps, &rp.job.board, &rp.job.epoch));
+    TRY(e->get("reg_abort", 1, &rp.abort));
+    CUDA_TRY(cudaMemsetAsync(rp.abort, 0, sizeof(int), e->stream));
+    CoopOrder& o = coop_order();
+    std::lock_guard<std::mutex> lock(o.m);
+    cudaEvent_t& done = o.done[e->device];
+    if (done == nullptr) CUDA_TRY(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
+    CUDA_TRY(cudaStreamWaitEvent(e->stream, done, 0));
+    const bool img = mode == 1 && P.floats_img <= region_max_floats();
+    const int rc = launch_regions(mode, img, P.plan->plan.pitch, rp, (int)P.plan->plan.blocks.size(), img ? P.floats_img : P.floats,
+                                  e->stream);
+    if (rc) return fail(PSDM_ERR_CUDA, "region launch: %s", cudaGetErrorString((cudaError_t)rc));
+    CUDA_TRY(cudaEventRecord(done, e->stream));
+    e->launches += 1;
+    return PSDM_OK;
+}
+
 // Buffers of the mixed-precision form (see below): FP32 staging of the
 // snapshots (slot m in stage[m % 4]; a snapshot is converted by the launch
 // after the one that stages it, and a launch of two steps may stage two),
@@ -925,6 +1112,18 @@ int launch_pairs(psdm_engine* e, int mode, const std::vector<PairArgs>& L) {
     return PSDM_OK;
 }
 
+// Receiver cells on the device, and the traces zeroed (a receiver in a cell
+// that no step updates keeps its zeros).
+int upload_receivers(psdm_engine* e, int nt, int nrec, const int* h_rec_cell, float* d_rec, const std::string& tag,
+                     int** d_rec_cell) {
+    *d_rec_cell = nullptr;
+    if (!d_rec || nrec <= 0) return PSDM_OK;
+    TRY(e->get(("rec_cell" + tag).c_str(), (size_t)nrec, d_rec_cell));
+    CUDA_TRY(cudaMemcpyAsync(*d_rec_cell, h_rec_cell, nrec * sizeof(int), cudaMemcpyHostToDevice, e->stream));
+    CUDA_TRY(cudaMemsetAsync(d_rec, 0, (size_t)nrec * nt * sizeof(float), e->stream));
+    return PSDM_OK;
+}
+
 // Step arguments of a forward pass over k = 2..nt
 // (solver_ac_forward_ram.f90:344-577).
 //   d_S: source trace (nt); d_fields: snapshot slots (nslots of ny*nx) or null;
@@ -941,11 +1140,7 @@ int build_forward(psdm_engine* e, Shot& s, int nt, int store_snap, const float* 
     int *d_row = nullptr, *d_cols = nullptr;
     TRY(upload_inj(e, g, inj, ("src" + tag).c_str(), &d_row, &d_cols));
     int* d_rec_cell = nullptr;
-    if (d_rec && nrec > 0) {
-        TRY(e->get(("rec_cell" + tag).c_str(), (size_t)nrec, &d_rec_cell));
-        CUDA_TRY(cudaMemcpyAsync(d_rec_cell, h_rec_cell, nrec * sizeof(int), cudaMemcpyHostToDevice, e->stream));
-        CUDA_TRY(cudaMemsetAsync(d_rec, 0, (size_t)nrec * nt * sizeof(float), e->stream));
-    }
+    TRY(upload_receivers(e, nt, nrec, h_rec_cell, d_rec, tag, &d_rec_cell));
     StepArgs a = base_args(s);
     plan_tiles(&a, inj.row_slot.data(), batched, true);
     a.row_slot = d_row;
@@ -975,11 +1170,58 @@ int build_forward(psdm_engine* e, Shot& s, int nt, int store_snap, const float* 
     return PSDM_OK;
 }
 
+// Forward pass as one region launch (build_forward's schedule).  Returns 1 if
+// the pass does not fit the form.
+int region_forward(psdm_engine* e, Shot& s, int nt, int store_snap, const float* d_S, int zs, int xs, float* d_fields,
+                   int nslots, int nrec, const int* h_rec_cell, float* d_rec) {
+    const Grid& g = s.g;
+    InjMap inj;
+    TRY(build_inj(g, 1, &zs, &xs, &inj));
+    const size_t fstride = g.field_cells();
+    std::vector<RegVar> var(nt - 1);
+    for (int k = 2; k <= nt; ++k) {
+        RegVar& v = var[k - 2];
+        v = RegVar{};
+        v.w = 1.f;
+        v.inj_t = k - 2;  // S(k-1)
+        v.inj_next = k < nt ? k - 1 : -1;
+        v.rec_t = (d_rec && k >= 3) ? k - 3 : -1;  // Rec(k-2) from level k-1
+        if (d_fields && (k - 1) % store_snap == 0) {
+            const int snap = (k - 1) / store_snap;  // 1-based slot
+            if (snap > nslots) return fail(PSDM_ERR_ARG, "snapshot slot %d exceeds nt_snap=%d", snap, nslots);
+            v.field = d_fields + (size_t)(snap - 1) * fstride;
+        }
+    }
+    RegPass P;
+    const int rc = region_prepare(e, s, inj, d_rec ? nrec : 0, h_rec_cell, var, "0", &P);
+    if (rc != PSDM_OK) return rc;
+    int* d_rec_cell = nullptr;
+    TRY(upload_receivers(e, nt, nrec, h_rec_cell, d_rec, "", &d_rec_cell));
+    StepArgs a = base_args(s);
+    a.inj_trace = d_S;
+    a.inj_ld = 0;
+    a.rec_out = d_rec;
+    a.rec_ld = nt;
+    set_buffers(s, 0, &a);
+    TRY(region_launch(e, 0, P, a, 0, nt - 1));
+    e->fwd_steps += nt - 1;
+    if (d_rec && nrec > 0) {
+        const int lr = launch_rec_final(d_rec_cell, s.p[(nt - 1) & 1], d_rec, nrec, nt, nt, e->stream);
+        if (lr) return fail(PSDM_ERR_CUDA, "receiver gather: %s", cudaGetErrorString((cudaError_t)lr));
+        e->launches += 1;
+    }
+    return PSDM_OK;
+}
+
 // Forward pass over k = 2..nt (solver_ac_forward_ram.f90:344-577).
 //   d_S: source trace (nt); d_fields: snapshot slots (nslots of ny*nx) or null;
 //   d_rec: receiver traces (NumRec, nt) or null.
 int run_forward(psdm_engine* e, Shot& s, int nt, int store_snap, const float* d_S, int zs, int xs,
                 float* d_fields, int nslots, int nrec, const int* h_rec_cell, float* d_rec) {
+    if (regions_on(e)) {
+        const int rc = region_forward(e, s, nt, store_snap, d_S, zs, xs, d_fields, nslots, nrec, h_rec_cell, d_rec);
+        if (rc != 1) return rc;
+    }
     std::vector<StepArgs> steps;
     std::vector<int> row_slot;
     TRY(build_forward(e, s, nt, store_snap, d_S, zs, xs, d_fields, nslots, nrec, h_rec_cell, d_rec, "", &steps, false,
@@ -1058,9 +1300,67 @@ int build_backward(psdm_engine* e, Shot& s, int nt, int store_snap, int nt_snap,
     return PSDM_OK;
 }
 
+// Snapshot slot read by each step of a backward pass over k = 2..nt, its
+// weight, or null (see build_backward).
+template <class F>
+void backward_slots(int nt, int store_snap, int nt_snap, int slot_lo, int slot_hi, const float* h_w, const F& fn) {
+    int snap = nt_snap;
+    for (int k = 2; k <= nt; ++k) {
+        int used = 0;
+        float w = 1.f;
+        if ((k - 1) % store_snap == 0) {
+            snap = snap - 1;
+            if (snap >= slot_lo && snap <= slot_hi && snap >= 1) {
+                w = h_w ? h_w[snap - 1] : 1.f;
+                if (w != 0.f) used = snap;  // a zero-padded slot contributes nothing
+            }
+        }
+        fn(k, used, w);
+    }
+}
+
+// Plain backward pass as one region launch.  Returns 1 if the pass does not
+// fit the form.
+int region_backward(psdm_engine* e, Shot& s, int nt, int store_snap, int nt_snap, const float* d_back, int reverse,
+                    int nrec, const int* zr, const int* xr, const float* d_fields, int slot_lo, int slot_hi,
+                    const float* h_w, float* d_image) {
+    const Grid& g = s.g;
+    InjMap inj;
+    TRY(build_inj(g, nrec, zr, xr, &inj));
+    const size_t fstride = g.field_cells();
+    std::vector<RegVar> var(nt - 1);
+    backward_slots(nt, store_snap, nt_snap, slot_lo, d_fields ? slot_hi : 0, h_w, [&](int k, int used, float w) {
+        RegVar& v = var[k - 2];
+        v = RegVar{};
+        v.w = used ? w : 1.f;
+        v.inj_t = reverse ? nt - k + 1 : k - 2;  // Sadj(k-1)
+        v.inj_next = k < nt ? (reverse ? nt - k : k - 1) : -1;
+        v.rec_t = -1;
+        if (used) v.field = const_cast<float*>(d_fields) + (size_t)(used - slot_lo) * fstride;
+        if (k > 2) var[k - 3].next = v.field;
+    });
+    RegPass P;
+    const int rc = region_prepare(e, s, inj, 0, nullptr, var, "1", &P);
+    if (rc != PSDM_OK) return rc;
+    StepArgs a = base_args(s);
+    a.inj_trace = d_back;
+    a.inj_ld = nt;
+    a.image = d_image;
+    a.ss = float(store_snap);
+    set_buffers(s, 0, &a);
+    TRY(region_launch(e, 1, P, a, 0, nt - 1));
+    e->bwd_steps += nt - 1;
+    return PSDM_OK;
+}
+
 int run_backward(psdm_engine* e, Shot& s, int nt, int store_snap, int nt_snap, const float* d_back, int reverse,
                  int nrec, const int* zr, const int* xr, const float* d_fields, int slot_lo, int slot_hi,
                  const float* h_w, float* d_image) {
+    if (regions_on(e)) {
+        const int rc = region_backward(e, s, nt, store_snap, nt_snap, d_back, reverse, nrec, zr, xr, d_fields, slot_lo,
+                                       slot_hi, h_w, d_image);
+        if (rc != 1) return rc;
+    }
     std::vector<StepArgs> steps;
     std::vector<int> row_slot;
     TRY(build_backward(e, s, nt, store_snap, nt_snap, d_back, reverse, nrec, zr, xr, d_fields, slot_lo, slot_hi, h_w,
@@ -2197,6 +2497,8 @@ int psdm_engine_destroy(psdm_engine* e) {
     for (cudaEvent_t ev : e->events) cudaEventDestroy(ev);
     for (cudaEvent_t ev : e->pass_staged)
         if (ev) cudaEventDestroy(ev);
+    for (auto& kv : e->reg_staged)
+        if (kv.second) cudaEventDestroy(kv.second);
     if (e->h_err) cudaFreeHost((void*)e->h_err);
     cudaStreamDestroy(e->own_stream);
     delete e;
@@ -2541,6 +2843,7 @@ int psdm_engine_set_pass_launch(psdm_engine* e, int32_t on) {
     TRY(check_engine(e));
     if (on < 0 || on > 2) return fail(PSDM_ERR_ARG, "pass launch form must be 0, 1 or 2 (got %d)", on);
     e->use_pass = on;
+    e->use_regions = false;
     return PSDM_OK;
 }
 

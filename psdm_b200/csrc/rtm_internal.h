@@ -413,6 +413,103 @@ int resident_blocks_per_sm(int mode, int sw);
 // Launch one pass (modes 0 and 1) of the resident kernel, rp.nreg blocks.
 int launch_resident(int mode, const ResParams& rp, void* stream);
 
+// ---- region pass kernel (rtm_region.cu) -------------------------------------
+// One cooperative launch per pass (of one shot, or of several shots side by
+// side), one block per region of the padded grid.
+#ifndef PSDM_REGION_THREADS
+#define PSDM_REGION_THREADS 384
+#endif
+constexpr int kRegThreads = PSDM_REGION_THREADS;
+constexpr int kRegPitches[2] = {72, 136};  // pitch of the shared columns: a region has at most pitch - 8 rows (fast)
+constexpr int kRegMaxQuads = 32;  // row quads of a region
+constexpr int kRegInterior = 0, kRegStrip = 1, kRegCorner = 2;
+// packet: shared offset | runs along the slow axis | of phi (corners) instead of p
+constexpr int kRegSlow = 1 << 30, kRegPhi = 1 << 29, kRegOffMask = kRegPhi - 1;
+// A region: nf x ns cells (fast, slow axes) from device row z0, column x0;
+// the fast axis is x if fastx, else z.
+struct RegBlock {
+    int type, fastx;
+    int low, lowf;  // the grid's edge lies on the low side of the slow (strips, corners) / fast (corners) axis
+    int z0, x0, nf, ns;
+    int P, Q;       // shared pitches with and without the ring
+    int nq;
+    // Inner cells, whose stencils end inside the region: row quads [qa, qb) x
+    // slow positions [sa, sb) (corners: fast positions [fa, fb)), in `items` items
+    // of C slow positions; the other quads or cells are the nbound boundary items.
+    int qa, qb, fa, fb, sa, sb, C, items, nbound;
+    int nslot;      // slots of the source buffer (set per pass)
+    int fsrow;      // fast position 0 is the free-surface row
+    int f0;         // interior: offset of its first cell in a pitched snapshot
+    int soff;       // corners: its first column within the corner
+    int pub0, npub, rcv0, nrcv, rcv_first;
+};
+// A region's share of one pass's geometry: its job, injection points
+// (RegParams::inj: offset in the region's source buffer, trace), the slots of
+// the row quads that hold them, and receivers (RegParams::rec: trace, shared offset).
+struct RegLoad {
+    int job, slot0, nslot, inj0, ninj, rec0, nrec, pad_;
+};
+// Values of one step.
+struct RegVar {
+    void* field;       // forward: FP32 snapshot written; backward: snapshot read (FP32, or 16-bit in mode 2); or null
+    void* aux;         // forward: largest |snapshot| (float bits) or null; mode 2: the snapshot's inverse scale
+    const void* next;  // backward: the next step's FP32 snapshot, or null
+    float w;           // taper weight of the snapshot
+    int inj_t;         // injection sample of this step
+    int inj_next;      // injection sample of the next step, or -1
+    int rec_t;         // receiver sample taken from level n at the start of this step, or -1
+};
+static_assert(sizeof(RegVar) % 8 == 0 && sizeof(RegVar) <= 128, "a warp fetches a RegVar");
+struct RegJob {
+    StepArgs a;         // arguments of the pass's first step
+    const RegVar* var;  // [nsteps]
+    void* board;        // 2 planes of npk 16-byte packets
+    int nsteps, npk;
+    unsigned int epoch; // tag of step i = epoch + i, used by no earlier launch on this board
+    int pad_;
+};
+struct RegPair {
+    int x, y;
+};
+struct RegParams {
+    RegJob job;             // the only job, or
+    const RegJob* jobs;     // several jobs (RegLoad::job); null for one
+    const RegBlock* blocks;
+    const RegLoad* loads;   // by block
+    const RegPair* pub;     // packets published: index, shared offset | kRegSlow
+    const int* rcv;         // packets received: shared offset | kRegSlow
+    const signed char* slots;
+    const RegPair* inj;
+    const RegPair* rec;
+    int* abort;             // device word, zero at launch
+    float neg0;             // -0: keeps packed products apart from the sums that take them
+};
+struct RegPlan {
+    std::vector<RegBlock> blocks;
+    std::vector<RegPair> pub;
+    std::vector<int> rcv;
+    int npk = 0, pitch = 0;
+    size_t floats = 0;  // shared floats of the largest region
+    double cost = 0;    // estimated cycles of a step
+};
+struct RegLists {
+    std::vector<RegLoad> loads;
+    std::vector<signed char> slots;
+    std::vector<RegPair> inj, rec;
+    size_t floats = 0, floats_img = 0;  // shared floats with the source buffers, and with the image
+};
+// Regions and packets of a padded grid for at most max_regions blocks of
+// max_floats shared floats.  False if the grid does not fit.
+bool plan_regions(const Grid& g, int fs, int max_regions, size_t max_floats, RegPlan* plan);
+// The regions' shares of a pass: injection points (linear cells x * ldz +
+// device row of interior cells, with their trace) and receivers.  False if
+// the source buffers do not fit.
+bool region_loads(const RegPlan& plan, const Grid& g, size_t max_floats, int ninj, const int* inj_cell,
+                  const int* inj_trace, int nrec, const int* rec_cell, RegLists* out);
+size_t region_max_floats();  // dynamic shared floats of a block (0 on failure)
+// img: the image of a plain backward pass stays in shared memory.
+int launch_regions(int mode, bool img, int pitch, const RegParams& rp, int nblocks, size_t floats, void* stream);
+
 // One kernel whose bounded copy wait runs out (nothing is copied); sets *err.
 int launch_wait_timeout_probe(int* err, void* stream);
 int launch_dt_quotients(float dt, float inv_dt, float div_lo, float div_hi, int fast_div, const float* x, float* q,

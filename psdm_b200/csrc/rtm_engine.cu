@@ -104,19 +104,20 @@ struct psdm_engine {
     // Until a launch form is chosen (psdm_engine_set_pass_launch), passes run
     // as one region launch each where the grid fits (rtm_region.cu).
     bool use_regions = true;
-    // Region plans by (ny, nx, dPML, fs, regions), each with its lists in
+    // Region plans by (ny, nx, dPML, fs, regions, pitch), each with its lists in
     // buffers of its own; the oldest gives way.
     struct RegSlot {
-        std::array<int, 5> key{};
+        std::array<int, 6> key{};
         bool used = false, fits = false;
         RegPlan plan;
         RegBlock* d_blocks = nullptr;
         RegPair* d_pub = nullptr;
         int* d_rcv = nullptr;
     };
-    static constexpr int kRegPlans = 12;
+    static constexpr int kRegPlans = 2 * kMaxSlots;
     RegSlot reg_plans[kRegPlans];
     int reg_next = 0;
+    std::map<std::array<int, 5>, double> reg_cost;  // region_step_cost by (ny, nx, dPML, fs, regions)
     std::map<std::string, cudaEvent_t> reg_staged;  // copies out of a staging buffer done
     unsigned int reg_epoch = 1;  // tag of the next region launch's first step
     void* reg_board = nullptr;   // the board whose tags reg_epoch counts
@@ -741,8 +742,8 @@ CoopOrder& coop_order() {
 
 // The plan of a grid for `regions` blocks, made and uploaded on first use.
 // *out = null if the grid does not fit.
-int region_plan(psdm_engine* e, const Grid& g, int fs, int regions, psdm_engine::RegSlot** out) {
-    const std::array<int, 5> key = {g.ny, g.nx, g.dPML, fs, regions};
+int region_plan(psdm_engine* e, const Grid& g, int fs, int regions, int pitch, psdm_engine::RegSlot** out) {
+    const std::array<int, 6> key = {g.ny, g.nx, g.dPML, fs, regions, pitch};
     *out = nullptr;
     for (auto& r : e->reg_plans)
         if (r.used && r.key == key) {
@@ -754,11 +755,12 @@ int region_plan(psdm_engine* e, const Grid& g, int fs, int regions, psdm_engine:
     e->reg_next = (k + 1) % psdm_engine::kRegPlans;
     r = psdm_engine::RegSlot{};
     r.key = key;
-    r.fits = plan_regions(g, fs, regions, region_max_floats(), &r.plan);
-    r.used = true;
-    if (!r.fits) return PSDM_OK;
+    r.fits = plan_regions(g, fs, regions, region_max_floats(), &r.plan, pitch);
+    if (!r.fits) {
+        r.used = true;
+        return PSDM_OK;
+    }
     const std::string t = std::to_string(k);
-    r.used = false;  // until the uploads are queued
     TRY(e->get(("reg_blocks" + t).c_str(), r.plan.blocks.size(), &r.d_blocks));
     TRY(e->get(("reg_pub" + t).c_str(), std::max<size_t>(r.plan.pub.size(), 1), &r.d_pub));
     TRY(e->get(("reg_rcv" + t).c_str(), std::max<size_t>(r.plan.rcv.size(), 1), &r.d_rcv));
@@ -768,54 +770,82 @@ int region_plan(psdm_engine* e, const Grid& g, int fs, int regions, psdm_engine:
                              e->stream));
     CUDA_TRY(cudaMemcpyAsync(r.d_rcv, r.plan.rcv.data(), r.plan.rcv.size() * sizeof(int), cudaMemcpyHostToDevice,
                              e->stream));
-    r.used = true;
+    r.used = true;  // once the uploads are queued
     *out = &r;
     return PSDM_OK;
 }
-
-// One pass of one shot as region launches: its plan, the device copies of its
-// geometry lists and per-step values.
-struct RegPass {
-    psdm_engine::RegSlot* plan = nullptr;
-    RegParams rp{};
-    size_t floats = 0, floats_img = 0;
-    RegVar* d_var = nullptr;
-    int nsteps = 0;
-};
 
 bool regions_on(const psdm_engine* e) {
     return e->use_regions && e->use_pass == 0 && e->steps_per_launch == 1 && region_max_floats() > 0;
 }
 
-// Prepare a pass: injection points by last write wins (build_inj's cells),
-// receivers, and the values of its steps.  `kind` names its buffers (passes
-// of different kinds may be queued together).  Returns 1 if the pass does not
-// fit the form.
-int region_prepare(psdm_engine* e, const Shot& s, const InjMap& inj, int nrec, const int* h_rec_cell,
-                   const std::vector<RegVar>& var, const std::string& kind, RegPass* P) {
-    const Grid& g = s.g;
-    TRY(region_plan(e, g, s.fs, e->num_sms, &P->plan));
-    if (!P->plan) return 1;
-    std::vector<int> cell, trace;
-    for (int zd = 0; zd < g.ldz; ++zd) {
-        if (inj.row_slot[zd] < 0) continue;
-        const int* c = inj.cols.data() + (size_t)inj.row_slot[zd] * g.nxt;
-        for (int x = 0; x < g.nxt; ++x)
-            if (c[x] >= 0) {
-                cell.push_back(x * g.ldz + zd);
-                trace.push_back(c[x]);
-            }
+// One pass of one shot, to be launched alone or beside other shots' passes.
+struct RegSpec {
+    Shot* s = nullptr;
+    psdm_engine::RegSlot* plan = nullptr;
+    InjMap inj;
+    int nrec = 0;
+    const int* h_rec_cell = nullptr;
+    std::vector<RegVar> var;  // its steps, from the shot's fresh state
+    StepArgs a;               // its arguments; a launch sets the buffers of its first step
+};
+
+// Prepared passes: the device copies of their geometry lists and step values.
+struct RegPass {
+    std::vector<RegSpec>* specs = nullptr;
+    std::vector<RegVar*> d_var;
+    RegParams rp;
+    int nblocks = 0, pitch = 0;
+    size_t floats = 0, floats_img = 0, npk = 0;
+};
+
+// Prepare passes that are launched together (specs with plans of one pitch).
+// `kind` names the buffers: passes of different kinds may be queued together.
+// Returns 1 if their injection points do not fit the form.
+int region_prepare(psdm_engine* e, std::vector<RegSpec>& specs, const std::string& kind, RegPass* P) {
+    std::memset(&P->rp, 0, sizeof P->rp);
+    P->specs = &specs;
+    P->pitch = specs[0].plan->plan.pitch;
+    RegLists all;
+    std::vector<RegVar> var;
+    std::vector<size_t> first;
+    for (size_t k = 0; k < specs.size(); ++k) {
+        RegSpec& sp = specs[k];
+        const Grid& g = sp.s->g;
+        std::vector<int> cell, trace;  // last write wins, as in build_inj's map
+        for (int zd = 0; zd < g.ldz; ++zd) {
+            if (sp.inj.row_slot[zd] < 0) continue;
+            const int* c = sp.inj.cols.data() + (size_t)sp.inj.row_slot[zd] * g.nxt;
+            for (int x = 0; x < g.nxt; ++x)
+                if (c[x] >= 0) {
+                    cell.push_back(x * g.ldz + zd);
+                    trace.push_back(c[x]);
+                }
+        }
+        RegLists L;
+        if (!region_loads(sp.plan->plan, g, region_max_floats(), (int)cell.size(), cell.data(), trace.data(), sp.nrec,
+                          sp.h_rec_cell, &L))
+            return 1;
+        for (RegLoad& l : L.loads) {
+            l.job = (int)k;
+            l.slot0 += (int)all.slots.size();
+            l.inj0 += (int)all.inj.size();
+            l.rec0 += (int)all.rec.size();
+        }
+        all.loads.insert(all.loads.end(), L.loads.begin(), L.loads.end());
+        all.slots.insert(all.slots.end(), L.slots.begin(), L.slots.end());
+        all.inj.insert(all.inj.end(), L.inj.begin(), L.inj.end());
+        all.rec.insert(all.rec.end(), L.rec.begin(), L.rec.end());
+        P->floats = std::max(P->floats, L.floats);
+        P->floats_img = std::max(P->floats_img, L.floats_img);
+        P->npk += (size_t)sp.plan->plan.npk;
+        first.push_back(var.size());
+        var.insert(var.end(), sp.var.begin(), sp.var.end());
     }
-    RegLists L;
-    if (!region_loads(P->plan->plan, g, region_max_floats(), (int)cell.size(), cell.data(), trace.data(), nrec,
-                      h_rec_cell, &L))
-        return 1;
-    P->floats = L.floats;
-    P->floats_img = L.floats_img;
-    P->nsteps = (int)var.size();
+    P->nblocks = (int)all.loads.size();
     // One staging buffer per kind, page-locked, refilled after its last copy.
-    const size_t nb[5] = {var.size() * sizeof(RegVar), L.loads.size() * sizeof(RegLoad),
-                          L.inj.size() * sizeof(RegPair), L.rec.size() * sizeof(RegPair), L.slots.size()};
+    const size_t nb[5] = {var.size() * sizeof(RegVar), all.loads.size() * sizeof(RegLoad),
+                          all.inj.size() * sizeof(RegPair), all.rec.size() * sizeof(RegPair), all.slots.size()};
     size_t off[6] = {0};
     for (int k = 0; k < 5; ++k) off[k + 1] = (off[k] + nb[k] + 15) & ~(size_t)15;
     char *h = nullptr, *d = nullptr;
@@ -824,18 +854,14 @@ int region_prepare(psdm_engine* e, const Shot& s, const InjMap& inj, int nrec, c
     CUDA_TRY(cudaEventSynchronize(done));
     TRY(e->get_pinned(("reg_stage" + kind).c_str(), off[5], reinterpret_cast<void**>(&h)));
     TRY(e->get(("reg_pass" + kind).c_str(), off[5], &d));
-    const void* src[5] = {var.data(), L.loads.data(), L.inj.data(), L.rec.data(), L.slots.data()};
+    const void* src[5] = {var.data(), all.loads.data(), all.inj.data(), all.rec.data(), all.slots.data()};
     for (int k = 0; k < 5; ++k)
         if (nb[k]) std::memcpy(h + off[k], src[k], nb[k]);
     CUDA_TRY(cudaMemcpyAsync(d, h, off[5], cudaMemcpyHostToDevice, e->stream));
     CUDA_TRY(cudaEventRecord(done, e->stream));
-    P->d_var = reinterpret_cast<RegVar*>(d);
+    for (size_t f : first) P->d_var.push_back(reinterpret_cast<RegVar*>(d) + f);
     RegParams& rp = P->rp;
-    rp.jobs = nullptr;
     rp.neg0 = -0.0f;
-    rp.blocks = P->plan->d_blocks;
-    rp.pub = P->plan->d_pub;
-    rp.rcv = P->plan->d_rcv;
     rp.loads = reinterpret_cast<const RegLoad*>(d + off[1]);
     rp.inj = reinterpret_cast<const RegPair*>(d + off[2]);
     rp.rec = reinterpret_cast<const RegPair*>(d + off[3]);
@@ -843,49 +869,61 @@ int region_prepare(psdm_engine* e, const Shot& s, const InjMap& inj, int nrec, c
     return PSDM_OK;
 }
 
-// The board of `npk` packets a plane and the tag of its next launch of
-// `nsteps` steps; tags never repeat on a board.
-int region_board(psdm_engine* e, size_t npk, int nsteps, void** board, unsigned int* epoch) {
-    const size_t bytes = std::max<size_t>(npk, 1) * 32;
-    char* b = nullptr;
-    TRY(e->get("reg_board", bytes, &b));
+void set_buffers(const Shot& s, int it, StepArgs* a);
+
+// Launch steps [i0, i1) of each prepared pass (none where i0 >= i1).
+int region_launch(psdm_engine* e, int mode, RegPass& P, const std::vector<std::pair<int, int>>& range) {
+    RegParams& rp = P.rp;
+    int most = 0;
+    for (auto& r : range) most = std::max(most, r.second - r.first);
+    if (most <= 0) return PSDM_OK;
+    // The board: 2 planes of packets for each pass; tags never repeat on it.
+    char* board = nullptr;
+    TRY(e->get("reg_board", std::max<size_t>(P.npk, 1) * 32, &board));
     const size_t have = e->bufs["reg_board"].bytes;
-    if (b != e->reg_board || have != e->reg_board_bytes || e->reg_epoch > 0xffffffffu - (unsigned int)nsteps - 1u) {
-        CUDA_TRY(cudaMemsetAsync(b, 0, have, e->stream));
-        e->reg_board = b;
+    if (board != e->reg_board || have != e->reg_board_bytes || e->reg_epoch > 0xffffffffu - (unsigned int)most - 1u) {
+        CUDA_TRY(cudaMemsetAsync(board, 0, have, e->stream));
+        e->reg_board = board;
         e->reg_board_bytes = have;
         e->reg_epoch = 1;
     }
-    *board = b;
-    *epoch = e->reg_epoch;
-    e->reg_epoch += (unsigned int)nsteps;
-    return PSDM_OK;
-}
-
-// Launch steps [i0, i1) of a prepared pass; `a` = the arguments of step i0.
-int region_launch(psdm_engine* e, int mode, RegPass& P, const StepArgs& a, int i0, int i1) {
-    if (i1 <= i0) return PSDM_OK;
-    RegParams& rp = P.rp;
-    rp.job = RegJob{};
-    rp.job.a = a;
-    rp.job.var = P.d_var + i0;
-    rp.job.nsteps = i1 - i0;
-    rp.job.npk = P.plan->plan.npk;
-    TRY(region_board(e, (size_t)rp.job.npk, rp.job.nsteps, &rp.job.board, &rp.job.epoch));
+    rp.epoch = e->reg_epoch;
+    e->reg_epoch += (unsigned int)most;
+    for (size_t k = 0; k < P.specs->size(); ++k) {
+        const RegSpec& sp = (*P.specs)[k];
+        RegJob& j = rp.job[k];
+        j.a = sp.a;
+        set_buffers(*sp.s, range[k].first, &j.a);
+        j.var = P.d_var[k] + range[k].first;
+        j.blocks = sp.plan->d_blocks;
+        j.pub = sp.plan->d_pub;
+        j.rcv = sp.plan->d_rcv;
+        j.board = board;
+        j.nsteps = std::max(0, range[k].second - range[k].first);
+        j.npk = sp.plan->plan.npk;
+        board += (size_t)j.npk * 32;
+    }
     TRY(e->get("reg_abort", 1, &rp.abort));
     CUDA_TRY(cudaMemsetAsync(rp.abort, 0, sizeof(int), e->stream));
+    const bool img = mode == 1 && P.floats_img <= region_max_floats();
     CoopOrder& o = coop_order();
     std::lock_guard<std::mutex> lock(o.m);
     cudaEvent_t& done = o.done[e->device];
     if (done == nullptr) CUDA_TRY(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
     CUDA_TRY(cudaStreamWaitEvent(e->stream, done, 0));
-    const bool img = mode == 1 && P.floats_img <= region_max_floats();
-    const int rc = launch_regions(mode, img, P.plan->plan.pitch, rp, (int)P.plan->plan.blocks.size(), img ? P.floats_img : P.floats,
-                                  e->stream);
+    const int rc =
+        launch_regions(mode, img, P.pitch, rp, P.nblocks, img ? P.floats_img : P.floats, e->stream);
     if (rc) return fail(PSDM_ERR_CUDA, "region launch: %s", cudaGetErrorString((cudaError_t)rc));
     CUDA_TRY(cudaEventRecord(done, e->stream));
     e->launches += 1;
     return PSDM_OK;
+}
+
+// Every step of each pass.
+int region_launch_all(psdm_engine* e, int mode, RegPass& P) {
+    std::vector<std::pair<int, int>> range;
+    for (const RegSpec& sp : *P.specs) range.push_back({0, (int)sp.var.size()});
+    return region_launch(e, mode, P, range);
 }
 
 // Buffers of the mixed-precision form (see below): FP32 staging of the
@@ -1170,18 +1208,16 @@ int build_forward(psdm_engine* e, Shot& s, int nt, int store_snap, const float* 
     return PSDM_OK;
 }
 
-// Forward pass as one region launch (build_forward's schedule).  Returns 1 if
-// the pass does not fit the form.
-int region_forward(psdm_engine* e, Shot& s, int nt, int store_snap, const float* d_S, int zs, int xs, float* d_fields,
-                   int nslots, int nrec, const int* h_rec_cell, float* d_rec) {
-    const Grid& g = s.g;
-    InjMap inj;
-    TRY(build_inj(g, 1, &zs, &xs, &inj));
-    const size_t fstride = g.field_cells();
-    std::vector<RegVar> var(nt - 1);
+// The forward pass of build_forward's schedule for the region form.
+int forward_spec(const Shot& s, int nt, int store_snap, const float* d_S, int zs, int xs, float* d_fields, int nslots,
+                 int nrec, const int* h_rec_cell, float* d_rec, RegSpec* sp) {
+    TRY(build_inj(s.g, 1, &zs, &xs, &sp->inj));
+    const size_t fstride = s.g.field_cells();
+    sp->nrec = d_rec ? nrec : 0;
+    sp->h_rec_cell = h_rec_cell;
+    sp->var.assign(nt - 1, RegVar{});
     for (int k = 2; k <= nt; ++k) {
-        RegVar& v = var[k - 2];
-        v = RegVar{};
+        RegVar& v = sp->var[k - 2];
         v.w = 1.f;
         v.inj_t = k - 2;  // S(k-1)
         v.inj_next = k < nt ? k - 1 : -1;
@@ -1192,18 +1228,29 @@ int region_forward(psdm_engine* e, Shot& s, int nt, int store_snap, const float*
             v.field = d_fields + (size_t)(snap - 1) * fstride;
         }
     }
+    sp->a = base_args(s);
+    sp->a.inj_trace = d_S;
+    sp->a.inj_ld = 0;
+    sp->a.rec_out = d_rec;
+    sp->a.rec_ld = nt;
+    return PSDM_OK;
+}
+
+// Forward pass as one region launch.  Returns 1 if the pass does not fit the
+// form.
+int region_forward(psdm_engine* e, Shot& s, int nt, int store_snap, const float* d_S, int zs, int xs, float* d_fields,
+                   int nslots, int nrec, const int* h_rec_cell, float* d_rec) {
+    std::vector<RegSpec> specs(1);
+    specs[0].s = &s;
+    TRY(region_plan(e, s.g, s.fs, e->num_sms, 0, &specs[0].plan));
+    if (!specs[0].plan) return 1;
+    TRY(forward_spec(s, nt, store_snap, d_S, zs, xs, d_fields, nslots, nrec, h_rec_cell, d_rec, &specs[0]));
     RegPass P;
-    const int rc = region_prepare(e, s, inj, d_rec ? nrec : 0, h_rec_cell, var, "0", &P);
+    const int rc = region_prepare(e, specs, "0", &P);
     if (rc != PSDM_OK) return rc;
     int* d_rec_cell = nullptr;
     TRY(upload_receivers(e, nt, nrec, h_rec_cell, d_rec, "", &d_rec_cell));
-    StepArgs a = base_args(s);
-    a.inj_trace = d_S;
-    a.inj_ld = 0;
-    a.rec_out = d_rec;
-    a.rec_ld = nt;
-    set_buffers(s, 0, &a);
-    TRY(region_launch(e, 0, P, a, 0, nt - 1));
+    TRY(region_launch_all(e, 0, P));
     e->fwd_steps += nt - 1;
     if (d_rec && nrec > 0) {
         const int lr = launch_rec_final(d_rec_cell, s.p[(nt - 1) & 1], d_rec, nrec, nt, nt, e->stream);
@@ -1319,36 +1366,48 @@ void backward_slots(int nt, int store_snap, int nt_snap, int slot_lo, int slot_h
     }
 }
 
-// Plain backward pass as one region launch.  Returns 1 if the pass does not
-// fit the form.
-int region_backward(psdm_engine* e, Shot& s, int nt, int store_snap, int nt_snap, const float* d_back, int reverse,
-                    int nrec, const int* zr, const int* xr, const float* d_fields, int slot_lo, int slot_hi,
-                    const float* h_w, float* d_image) {
-    const Grid& g = s.g;
-    InjMap inj;
-    TRY(build_inj(g, nrec, zr, xr, &inj));
-    const size_t fstride = g.field_cells();
-    std::vector<RegVar> var(nt - 1);
+// The plain backward pass of build_backward's schedule for the region form.
+// slot_of_step (optional): the snapshot slot each step images, 0 for none.
+int backward_spec(const Shot& s, int nt, int store_snap, int nt_snap, const float* d_back, int reverse, int nrec,
+                  const int* zr, const int* xr, const float* d_fields, int slot_lo, int slot_hi, const float* h_w,
+                  float* d_image, RegSpec* sp, std::vector<int>* slot_of_step = nullptr) {
+    TRY(build_inj(s.g, nrec, zr, xr, &sp->inj));
+    const size_t fstride = s.g.field_cells();
+    sp->var.assign(nt - 1, RegVar{});
+    std::vector<RegVar>& var = sp->var;
     backward_slots(nt, store_snap, nt_snap, slot_lo, d_fields ? slot_hi : 0, h_w, [&](int k, int used, float w) {
         RegVar& v = var[k - 2];
-        v = RegVar{};
         v.w = used ? w : 1.f;
         v.inj_t = reverse ? nt - k + 1 : k - 2;  // Sadj(k-1)
         v.inj_next = k < nt ? (reverse ? nt - k : k - 1) : -1;
         v.rec_t = -1;
         if (used) v.field = const_cast<float*>(d_fields) + (size_t)(used - slot_lo) * fstride;
         if (k > 2) var[k - 3].next = v.field;
+        if (slot_of_step) slot_of_step->push_back(used);
     });
+    sp->a = base_args(s);
+    sp->a.inj_trace = d_back;
+    sp->a.inj_ld = nt;
+    sp->a.image = d_image;
+    sp->a.ss = float(store_snap);
+    return PSDM_OK;
+}
+
+// Plain backward pass as one region launch.  Returns 1 if the pass does not
+// fit the form.
+int region_backward(psdm_engine* e, Shot& s, int nt, int store_snap, int nt_snap, const float* d_back, int reverse,
+                    int nrec, const int* zr, const int* xr, const float* d_fields, int slot_lo, int slot_hi,
+                    const float* h_w, float* d_image) {
+    std::vector<RegSpec> specs(1);
+    specs[0].s = &s;
+    TRY(region_plan(e, s.g, s.fs, e->num_sms, 0, &specs[0].plan));
+    if (!specs[0].plan) return 1;
+    TRY(backward_spec(s, nt, store_snap, nt_snap, d_back, reverse, nrec, zr, xr, d_fields, slot_lo, slot_hi, h_w,
+                      d_image, &specs[0]));
     RegPass P;
-    const int rc = region_prepare(e, s, inj, 0, nullptr, var, "1", &P);
+    const int rc = region_prepare(e, specs, "1", &P);
     if (rc != PSDM_OK) return rc;
-    StepArgs a = base_args(s);
-    a.inj_trace = d_back;
-    a.inj_ld = nt;
-    a.image = d_image;
-    a.ss = float(store_snap);
-    set_buffers(s, 0, &a);
-    TRY(region_launch(e, 1, P, a, 0, nt - 1));
+    TRY(region_launch_all(e, 1, P));
     e->bwd_steps += nt - 1;
     return PSDM_OK;
 }
@@ -1525,6 +1584,86 @@ void mixed_backward_args(const MixedBufs& mb, int nt, const float* h_w, std::vec
     }
 }
 
+// ---- the mixed form as region launches
+//
+// A snapshot's scale needs its largest magnitude over the whole grid, which
+// regions that run ahead of one another do not have.  The forward pass
+// therefore stages up to nstage FP32 snapshots with their magnitudes in one
+// launch, and a conversion launch follows: with 512 MB of staging a 1200 x
+// 1136 window pauses every 384 steps at ks = 4, under 2 % of the pass.
+
+// Snapshots staged by one launch: `bytes` of staging, an eighth of the free
+// memory at most; 0 when there is no room for a few.
+int mixed_stage(psdm_engine* e, size_t fstride, int nsnap, size_t bytes, const std::string& tag, float** stage,
+                int* nstage) {
+    *nstage = 0;
+    size_t fr = 0, tot = 0;
+    CUDA_TRY(cudaMemGetInfo(&fr, &tot));
+    const size_t have = e->bufs[("reg_staging" + tag)].bytes;
+    const size_t room = std::max(have, std::min(bytes, fr / 8));
+    const int n = (int)std::min<size_t>(room / (fstride * sizeof(float)), (size_t)std::max(nsnap, 1));
+    if (n < std::min(4, std::max(nsnap, 1))) return PSDM_OK;
+    TRY(e->get(("reg_staging" + tag).c_str(), fstride * (size_t)n, stage));
+    *nstage = n;
+    return PSDM_OK;
+}
+
+void mixed_forward_vars(const MixedBufs& mb, float* stage, int nstage, std::vector<RegVar>& var) {
+    for (int m = 1; m <= mb.nsnap; ++m) {
+        RegVar& v = var[(size_t)m * mb.ks - 1];  // step k = ks m + 1
+        v.field = stage + (size_t)((m - 1) % nstage) * mb.fstride;
+        v.aux = mb.amax + (m - 1);
+    }
+}
+
+void mixed_backward_vars(const MixedBufs& mb, int nt, const float* h_w, RegSpec* sp) {
+    for (int k = 2; k <= nt; ++k) {
+        RegVar& v = sp->var[k - 2];
+        v.field = v.aux = nullptr;
+        v.next = nullptr;
+        v.w = 1.f;
+        const int r = nt + 1 - k;
+        if (r % mb.ks != 0) continue;
+        const int m = r / mb.ks;
+        if (m < 1 || m > mb.nsnap) continue;
+        const float w = h_w ? h_w[(size_t)mb.ks * m - 1] : 1.f;
+        if (w == 0.f) continue;  // zero weight: no contribution
+        v.field = mb.snap16 + (size_t)(m - 1) * mb.fstride;
+        v.aux = mb.iscale + (m - 1);
+        v.w = w;
+    }
+    sp->a.kind16 = mb.kind;
+    sp->a.comp = mb.comp;
+    sp->a.ss = float(mb.ks);
+}
+
+// Forward passes of the mixed form: launches of up to nstage snapshots each,
+// every one followed by the conversion of what it staged.
+int region_mixed_forward(psdm_engine* e, RegPass& P, const std::vector<const MixedBufs*>& mb,
+                         const std::vector<float*>& stage, int nstage) {
+    const size_t n = P.specs->size();
+    std::vector<std::pair<int, int>> range(n, {0, 0});
+    for (int c = 0;; ++c) {
+        bool any = false;
+        for (size_t k = 0; k < n; ++k) {
+            const int steps = (int)(*P.specs)[k].var.size(), m1 = std::min((c + 1) * nstage, mb[k]->nsnap);
+            range[k].first = range[k].second;
+            range[k].second = m1 == mb[k]->nsnap ? steps : m1 * mb[k]->ks;
+            any = any || range[k].second > range[k].first;
+        }
+        if (!any) return PSDM_OK;
+        TRY(region_launch(e, 0, P, range));
+        for (size_t k = 0; k < n; ++k) {
+            const int m0 = std::min(c * nstage, mb[k]->nsnap), cnt = std::min((c + 1) * nstage, mb[k]->nsnap) - m0;
+            if (cnt <= 0) continue;
+            const int rc = launch_quantize_many(stage[k], mb[k]->amax + m0, mb[k]->snap16 + (size_t)m0 * mb[k]->fstride,
+                                                mb[k]->iscale + m0, (int)mb[k]->fstride, mb[k]->kind, cnt, e->stream);
+            if (rc) return fail(PSDM_ERR_CUDA, "snapshot conversion launch: %s", cudaGetErrorString((cudaError_t)rc));
+            e->launches += 1;
+        }
+    }
+}
+
 // Per-sample taper weights of the snapshot series (calculate_PSDM_RTM.f90:421-427).
 std::vector<float> taper_weights(int nt_prop2, int nt_taper, int taper_option, int N_taper, int N_zeros) {
     std::vector<float> wts(std::max(nt_taper, 1), 1.f);
@@ -1584,6 +1723,77 @@ int launch_direct(psdm_engine* e, int mode, const StepArgs& a) {
     return PSDM_OK;
 }
 
+// The checkpointed shot as region launches, one per segment of each pass.  The
+// last segment keeps its snapshots the first time it runs, so the forward
+// pass runs once more for the other segments only.  Returns 1, before
+// anything is launched, if the passes do not fit the form.
+int region_shot_checkpointed(psdm_engine* e, Shot& f, Shot& b, int NumRec, const WinGeom& w, const float* d_S,
+                             const float* d_tgt, int store_snap, int nt_prop2, int nt_taper, const float* wts, int K,
+                             float* segbuf, float* ckpts, float* d_imgp) {
+    const size_t fstride = f.g.field_cells(), sf = state_floats(f);
+    const int nsteps = nt_prop2 - 1, nseg = (nsteps + K - 1) / K, nsnap = nsteps / store_snap;
+    std::vector<RegSpec> fw(1), re(1), bw(1);
+    fw[0].s = re[0].s = &f;
+    bw[0].s = &b;
+    TRY(region_plan(e, f.g, f.fs, e->num_sms, 0, &fw[0].plan));
+    if (!fw[0].plan) return 1;
+    re[0].plan = bw[0].plan = fw[0].plan;
+    TRY(forward_spec(f, nt_prop2, store_snap, d_S, w.zs, w.xs, nullptr, 0, 0, nullptr, nullptr, &fw[0]));
+    TRY(forward_spec(f, nt_prop2, store_snap, d_S, w.zs, w.xs, nullptr, 0, 0, nullptr, nullptr, &re[0]));
+    for (int t = 0; t < nsteps; ++t)  // the snapshot of step t, in its segment's slot
+        if ((t + 1) % store_snap == 0 && (t + 1) / store_snap <= nsnap)
+            re[0].var[t].field = segbuf + (size_t)(t % K) * fstride;
+    std::vector<int> slot;
+    TRY(backward_spec(b, nt_taper, store_snap, nt_taper, d_tgt, 1, NumRec, w.zr.data(), w.xr.data(), segbuf, 1, nsnap,
+                      wts, d_imgp, &bw[0], &slot));
+    for (size_t i = 0; i < slot.size(); ++i) {
+        RegVar& v = bw[0].var[i];
+        v.field = slot[i] > 0 ? segbuf + (size_t)((store_snap * slot[i] - 1) % K) * fstride : nullptr;
+        v.next = nullptr;  // set below within a segment
+    }
+    auto segment = [&](size_t i) { return slot[i] > 0 ? (store_snap * slot[i] - 1) / K : -1; };
+    for (size_t i = 0; i + 1 < slot.size(); ++i)
+        if (segment(i) >= 0 && segment(i) == segment(i + 1)) bw[0].var[i].next = bw[0].var[i + 1].field;
+    RegPass F, R, B;
+    int rc = region_prepare(e, fw, "c0", &F);
+    if (rc == PSDM_OK) rc = region_prepare(e, re, "c1", &R);
+    if (rc == PSDM_OK) rc = region_prepare(e, bw, "c2", &B);
+    if (rc != PSDM_OK) return rc;
+    for (int j = 0; j < nseg; ++j) {
+        if (j > 0) TRY(copy_state(e, f, ckpts + sf * (size_t)(j - 1), true));
+        TRY(region_launch(e, 0, j + 1 < nseg ? F : R, {{j * K, std::min((j + 1) * K, nsteps)}}));
+    }
+    e->fwd_steps += nsteps;
+    TRY(e->record(1));
+    CUDA_TRY(cudaMemsetAsync(d_imgp, 0, fstride * sizeof(float), e->stream));
+    int cur = nseg - 1;  // segment whose snapshots segbuf holds
+    for (size_t i = 0; i < slot.size();) {
+        // steps up to the next one that needs another segment
+        size_t i1 = i;
+        int need = -1;
+        for (; i1 < slot.size(); ++i1) {
+            const int g = segment(i1);
+            if (g < 0) continue;
+            if (need < 0) need = g;
+            if (g != need) break;
+        }
+        if (need >= 0 && need != cur) {
+            if (need == 0)
+                TRY(reset_state(e, &f));
+            else
+                TRY(copy_state(e, f, ckpts + sf * (size_t)(need - 1), false));
+            const int r1 = std::min((need + 1) * K, nsteps);
+            TRY(region_launch(e, 0, R, {{need * K, r1}}));
+            e->fwd_steps += r1 - need * K;
+            cur = need;
+        }
+        TRY(region_launch(e, 1, B, {{(int)i, (int)i1}}));
+        i = i1;
+    }
+    e->bwd_steps += (int64_t)slot.size();
+    return e->record(2);
+}
+
 int rtm_shot_checkpointed(psdm_engine* e, const psdm_params* prm, int NumRec, int nxSou, int nySou, const int* nxRec,
                           const int* nyRec, const float* d_S, const float* d_tgt, float dd, float dt, int ny, int nx,
                           int nx_w, const float* d_vp, float added_space, int store_snap, int nt_prop2, int nt_taper,
@@ -1604,6 +1814,16 @@ int rtm_shot_checkpointed(psdm_engine* e, const psdm_params* prm, int NumRec, in
     if (nseg > 1) TRY(e->get("ck_states", sf * (size_t)(nseg - 1), &ckpts));
     TRY(e->get("image_pitched", fstride, &d_imgp));
     TRY(e->record(0));
+    if (regions_on(e)) {
+        const int rc = region_shot_checkpointed(e, f, b, NumRec, w, d_S, d_tgt, store_snap, nt_prop2, nt_taper, wts,
+                                                K, segbuf, ckpts, d_imgp);
+        if (rc != 1) {
+            TRY(rc);
+            CUDA_TRY(cudaMemcpy2DAsync(d_img, (size_t)ny * sizeof(float), d_imgp, (size_t)b.g.ldf * sizeof(float),
+                                       (size_t)ny * sizeof(float), nx_w, cudaMemcpyDeviceToDevice, e->stream));
+            return PSDM_OK;
+        }
+    }
     // Forward steps: without snapshots (first pass), and with the snapshot
     // of step k in segment slot (k-2) % K (recomputation).
     std::vector<StepArgs> fwd;
@@ -1764,6 +1984,38 @@ int rtm_shot_mixed_ckpt(psdm_engine* e, const psdm_params* prm, int NumRec, int 
                         int nx_w, const float* d_vp, float added_space, int store_snap, int nt_prop2, int nt_taper,
                         int taper_option, int N_taper, int N_zeros, float* d_img);
 
+// Both passes of a mixed-precision shot as region launches.  Returns 1,
+// before anything is launched, if they do not fit the form.
+int region_mixed_shot(psdm_engine* e, Shot& s, const MixedBufs& mb, int NumRec, const WinGeom& w, const float* d_S,
+                      const float* d_tgt, int store_snap, int nt_prop2, int nt_taper, const float* wts, float* d_imgp) {
+    std::vector<RegSpec> fw(1), bw(1);
+    fw[0].s = bw[0].s = &s;
+    TRY(region_plan(e, s.g, s.fs, e->num_sms, 0, &fw[0].plan));
+    if (!fw[0].plan) return 1;
+    bw[0].plan = fw[0].plan;
+    float* stage = nullptr;
+    int nstage = 0;
+    TRY(mixed_stage(e, mb.fstride, mb.nsnap, (size_t)512 << 20, "", &stage, &nstage));
+    if (nstage == 0) return 1;
+    TRY(forward_spec(s, nt_prop2, store_snap, d_S, w.zs, w.xs, nullptr, 0, 0, nullptr, nullptr, &fw[0]));
+    mixed_forward_vars(mb, stage, nstage, fw[0].var);
+    TRY(backward_spec(s, nt_taper, store_snap, nt_taper, d_tgt, 1, NumRec, w.zr.data(), w.xr.data(), nullptr, 1, 0,
+                      nullptr, d_imgp, &bw[0]));
+    mixed_backward_vars(mb, nt_taper, wts, &bw[0]);
+    RegPass F, B;
+    int rc = region_prepare(e, fw, "0", &F);
+    if (rc == PSDM_OK) rc = region_prepare(e, bw, "1", &B);
+    if (rc != PSDM_OK) return rc;
+    TRY(region_mixed_forward(e, F, {&mb}, {stage}, nstage));
+    e->fwd_steps += nt_prop2 - 1;
+    TRY(e->record(1));
+    CUDA_TRY(cudaMemsetAsync(d_imgp, 0, mb.fstride * sizeof(float), e->stream));
+    TRY(reset_state(e, &s));
+    TRY(region_launch_all(e, 2, B));
+    e->bwd_steps += nt_taper - 1;
+    return e->record(2);
+}
+
 int rtm_shot_core(psdm_engine* e, const psdm_params* prm, int NumRec, int nxSou, int nySou, const int* nxRec,
                   const int* nyRec, const float* d_S, const float* d_tgt, float dd, float dt, int ny, int nx,
                   int nx_w, const float* d_vp, float added_space, int store_snap, int nt_snap, int nt_prop2,
@@ -1794,6 +2046,17 @@ int rtm_shot_core(psdm_engine* e, const psdm_params* prm, int NumRec, int nxSou,
         MixedBufs mb;
         TRY(mixed_bufs(e, s, prm->precision, store_snap, nt_prop2, "", &mb));
         TRY(e->record(0));
+        if (regions_on(e)) {
+            const std::vector<float> wts = taper_weights(nt_prop2, nt_taper, taper_option, N_taper, N_zeros);
+            const int rc = region_mixed_shot(e, s, mb, NumRec, w, d_S, d_tgt, store_snap, nt_prop2, nt_taper,
+                                             wts.data(), d_imgp);
+            if (rc != 1) {
+                TRY(rc);
+                CUDA_TRY(cudaMemcpy2DAsync(d_img, (size_t)ny * sizeof(float), d_imgp, (size_t)s.g.ldf * sizeof(float),
+                                           (size_t)ny * sizeof(float), nx_w, cudaMemcpyDeviceToDevice, e->stream));
+                return PSDM_OK;
+            }
+        }
         std::vector<StepArgs> fw;
         std::vector<int> row_slot;
         TRY(build_forward(e, s, nt_prop2, store_snap, d_S, w.zs, w.xs, nullptr, 0, 0, nullptr, nullptr, "", &fw,
@@ -2143,12 +2406,16 @@ int batch_program_ckpt(psdm_engine* e, const BatchJob& j, BatchSlot& sl, int i, 
     return PSDM_OK;
 }
 
-int batch_start(psdm_engine* e, const BatchJob& j, BatchSlot& sl, int i) {
+// Shot `i`'s inputs, state and window in slot `sl`.
+int batch_inputs(psdm_engine* e, const BatchJob& j, BatchSlot& sl, int i, const float** p_vp, const float** p_tgt,
+                 WinGeom* w) {
     const psdm_shot& sh = j.shots[i];
     const int ny = j.ny, nx_w = sh.nx_w;
     const std::string& tag = sl.tag;
-    const float* d_vp = sh.Vp_w;
-    const float* d_tgt = sh.Data_target;
+    const float*& d_vp = *p_vp;
+    const float*& d_tgt = *p_tgt;
+    d_vp = sh.Vp_w;
+    d_tgt = sh.Data_target;
     const size_t nvp = (size_t)ny * nx_w, ntgt = (size_t)sh.NumRec * sh.nt_taper;
     // The slot's page-locked staging is reused only once its previous
     // copies have completed.
@@ -2167,24 +2434,31 @@ int batch_start(psdm_engine* e, const BatchJob& j, BatchSlot& sl, int i) {
         d_tgt = dtg;
     }
     TRY(setup_shot(e, j.prm, ny, nx_w, j.dd, j.dt, d_vp, &sl.s, tag));
-    WinGeom w;
-    TRY(window_geometry(sl.s.g, sh.NumRec, sh.nxSou, sh.nySou, sh.nxRec, sh.nyRec, j.dd, j.nx, j.added_space, &w));
-    if (w.nx_w_calc != nx_w)
+    TRY(window_geometry(sl.s.g, sh.NumRec, sh.nxSou, sh.nySou, sh.nxRec, sh.nyRec, j.dd, j.nx, j.added_space, w));
+    if (w->nx_w_calc != nx_w)
         return fail(PSDM_ERR_ARG, "shot %d: nx_w=%d does not match the window of its geometry (%d)", i, nx_w,
-                    w.nx_w_calc);
-    if (e->ckpt_interval > 0)
-        TRY(batch_program_ckpt(e, j, sl, i, w, d_vp, d_tgt, e->ckpt_interval));
-    else
-        TRY(batch_program_plain(e, j, sl, i, w, d_tgt));
-    const size_t fstride = sl.s.g.field_cells();
-    CUDA_TRY(cudaEventRecord(sl.staged, e->stream));
-    CUDA_TRY(cudaMemsetAsync(sl.d_imgp, 0, fstride * sizeof(float), e->stream));
+                    w->nx_w_calc);
     sl.shot = i;
     sl.pc = 0;
     sl.out_ny = ny;
     sl.out_nx = nx_w;
     sl.d_out = j.host_io ? nullptr : sh.PSDM_w;
     sl.h_out = nullptr;
+    return PSDM_OK;
+}
+
+int batch_start(psdm_engine* e, const BatchJob& j, BatchSlot& sl, int i) {
+    const float *d_vp = nullptr, *d_tgt = nullptr;
+    WinGeom w;
+    TRY(batch_inputs(e, j, sl, i, &d_vp, &d_tgt, &w));
+    sl.shot = -1;  // until its program is ready
+    if (e->ckpt_interval > 0)
+        TRY(batch_program_ckpt(e, j, sl, i, w, d_vp, d_tgt, e->ckpt_interval));
+    else
+        TRY(batch_program_plain(e, j, sl, i, w, d_tgt));
+    CUDA_TRY(cudaEventRecord(sl.staged, e->stream));
+    CUDA_TRY(cudaMemsetAsync(sl.d_imgp, 0, sl.s.g.field_cells() * sizeof(float), e->stream));
+    sl.shot = i;
     return PSDM_OK;
 }
 
@@ -2214,6 +2488,152 @@ int batch_finish(psdm_engine* e, const BatchJob& j, BatchSlot& sl) {
     } else {
         CUDA_TRY(cudaMemcpy2DAsync(sl.d_out, row, sl.d_imgp, ld, row, sl.out_nx, cudaMemcpyDeviceToDevice,
                                    e->stream));
+    }
+    return PSDM_OK;
+}
+
+// ---- batched shots as region launches
+//
+// Shots whose grids fit the region form run in groups, every shot of a group
+// on its own share of the multiprocessors, one launch for the group's forward
+// passes and one for its backward passes.  A step of a small grid is bound by
+// its chain of latencies, so several run side by side in the time of one; a
+// grid that fills the device runs alone.
+
+// Cells times steps of a shot, its share of a group's multiprocessors.
+double batch_weight(const BatchJob& j, const psdm_shot& sh) {
+    const Grid g = make_grid(j.prm->dPML, j.ny, sh.nx_w);
+    return (double)g.nyt * g.nxt * ((double)sh.nt_prop2 + sh.nt_taper);
+}
+
+// Multiprocessors of each shot of a group, in proportion to their work.
+std::vector<int> batch_shares(const psdm_engine* e, const BatchJob& j, int first, int n) {
+    std::vector<double> w;
+    double sum = 0;
+    for (int k = 0; k < n; ++k) {
+        w.push_back(batch_weight(j, j.shots[first + k]));
+        sum += w.back();
+    }
+    std::vector<int> r(n);
+    for (int k = 0; k < n; ++k) r[k] = std::max(1, (int)(e->num_sms * w[k] / sum));
+    return r;
+}
+
+// Estimated step of a grid on `regions` multiprocessors; < 0 if it does not fit.
+double batch_step_cost(psdm_engine* e, const Grid& g, int fs, int regions) {
+    const std::array<int, 5> key = {g.ny, g.nx, g.dPML, fs, regions};
+    auto it = e->reg_cost.find(key);
+    if (it == e->reg_cost.end()) {
+        if (e->reg_cost.size() > 256) e->reg_cost.clear();
+        it = e->reg_cost.emplace(key, region_step_cost(g, fs, regions, region_max_floats())).first;
+    }
+    return it->second;
+}
+
+// Shots of the group that starts at `first`: the size with the least
+// estimated time a shot, of at most `most`; 0 if the first shot does not fit.
+int batch_group(psdm_engine* e, const BatchJob& j, int first, int most) {
+    int best = 0;
+    double best_t = 0;
+    for (int n = 1; n <= most && first + n <= j.nshots; ++n) {
+        const std::vector<int> share = batch_shares(e, j, first, n);
+        double t = 0;
+        for (int k = 0; k < n && t >= 0; ++k) {
+            const psdm_shot& sh = j.shots[first + k];
+            const double c = batch_step_cost(e, make_grid(j.prm->dPML, j.ny, sh.nx_w), j.prm->fs != 0, share[k]);
+            t = c < 0 ? -1.0 : std::max(t, c * ((double)sh.nt_prop2 + sh.nt_taper));
+        }
+        if (t < 0) {
+            if (n == 1) return 0;
+            break;
+        }
+        if (best == 0 || t / n < best_t) {
+            best = n;
+            best_t = t / n;
+        } else if (n > 2 * best) {
+            break;
+        }
+    }
+    return best;
+}
+
+// The group of n shots from `first` in slots[0..n).  Returns 1, before a pass
+// is launched, if one of them does not fit.
+int batch_group_run(psdm_engine* e, const BatchJob& j, std::vector<BatchSlot>& slots, int first, int n) {
+    const bool mixed = j.prm->precision != PSDM_PREC_FP32;
+    const std::vector<int> share = batch_shares(e, j, first, n);
+    std::vector<RegSpec> fw(n), bw(n);
+    std::vector<float*> stage(n, nullptr);
+    std::vector<const MixedBufs*> mb(n);
+    int nstage = 1 << 30, pitch = 0;
+    for (int k = 0; k < n; ++k) {
+        BatchSlot& sl = slots[k];
+        const psdm_shot& sh = j.shots[first + k];
+        TRY(batch_flush(e, sl));
+        const float *d_vp = nullptr, *d_tgt = nullptr;
+        WinGeom w;
+        TRY(batch_inputs(e, j, sl, first + k, &d_vp, &d_tgt, &w));
+        const Grid& g = sl.s.g;
+        const size_t fstride = g.field_cells();
+        const int nsnap = (sh.nt_prop2 - 1) / j.store_snap;
+        TRY(region_plan(e, g, sl.s.fs, share[k], pitch, &fw[k].plan));
+        if (!fw[k].plan) return 1;
+        pitch = fw[k].plan->plan.pitch;
+        float* d_F = nullptr;
+        if (mixed) {
+            TRY(mixed_bufs(e, sl.s, j.prm->precision, j.store_snap, sh.nt_prop2, sl.tag, &sl.mb));
+            int ns = 0;
+            TRY(mixed_stage(e, fstride, nsnap, ((size_t)512 << 20) / n, sl.tag, &stage[k], &ns));
+            if (ns == 0) return 1;
+            nstage = std::min(nstage, ns);
+        } else if (nsnap > 0) {
+            TRY(e->get(("fields" + sl.tag).c_str(), fstride * nsnap, &d_F));
+        }
+        TRY(e->get(("imgp" + sl.tag).c_str(), fstride, &sl.d_imgp));
+        CUDA_TRY(cudaMemsetAsync(sl.d_imgp, 0, fstride * sizeof(float), e->stream));
+        const std::vector<float> wts = taper_weights(sh.nt_prop2, sh.nt_taper, j.taper_option, j.N_taper, j.N_zeros);
+        fw[k].s = bw[k].s = &sl.s;
+        bw[k].plan = fw[k].plan;
+        TRY(forward_spec(sl.s, sh.nt_prop2, j.store_snap, j.d_S, w.zs, w.xs, d_F, nsnap, 0, nullptr, nullptr, &fw[k]));
+        TRY(backward_spec(sl.s, sh.nt_taper, j.store_snap, sh.nt_taper, d_tgt, 1, sh.NumRec, w.zr.data(), w.xr.data(),
+                          d_F, 1, nsnap, wts.data(), sl.d_imgp, &bw[k]));
+        if (mixed) mixed_backward_vars(sl.mb, sh.nt_taper, wts.data(), &bw[k]);
+        mb[k] = &sl.mb;
+        if (j.host_io) CUDA_TRY(cudaEventRecord(sl.staged, e->stream));
+    }
+    if (mixed)
+        for (int k = 0; k < n; ++k) mixed_forward_vars(*mb[k], stage[k], nstage, fw[k].var);
+    RegPass F, B;
+    int rc = region_prepare(e, fw, "0", &F);
+    if (rc == PSDM_OK) rc = region_prepare(e, bw, "1", &B);
+    if (rc != PSDM_OK) return rc;
+    if (mixed)
+        TRY(region_mixed_forward(e, F, mb, stage, nstage));
+    else
+        TRY(region_launch_all(e, 0, F));
+    for (int k = 0; k < n; ++k) TRY(reset_state(e, &slots[k].s));  // second propagator call: fresh wavefield
+    TRY(region_launch_all(e, mixed ? 2 : 1, B));
+    for (int k = 0; k < n; ++k) {
+        e->fwd_steps += (int64_t)fw[k].var.size();
+        e->bwd_steps += (int64_t)bw[k].var.size();
+        TRY(batch_finish(e, j, slots[k]));
+        slots[k].shot = -1;
+    }
+    return PSDM_OK;
+}
+
+// The shots from the first one on in groups, up to one whose grid or
+// injection points do not fit the form; *done = shots run.
+int run_batch_regions(psdm_engine* e, const BatchJob& j, std::vector<BatchSlot>& slots, int* done) {
+    for (*done = 0; *done < j.nshots;) {
+        const psdm_shot& sh = j.shots[*done];
+        if (sh.nx_w < 1 || j.ny < 1) return PSDM_OK;  // refused where the shot starts
+        int n = batch_group(e, j, *done, (int)slots.size());
+        int rc = n > 0 ? batch_group_run(e, j, slots, *done, n) : 1;
+        if (rc == 1 && n > 1) rc = batch_group_run(e, j, slots, *done, n = 1);
+        for (BatchSlot& sl : slots) sl.shot = -1;
+        if (rc != PSDM_OK) return rc == 1 ? PSDM_OK : rc;
+        *done += n;
     }
     return PSDM_OK;
 }
@@ -2285,6 +2705,9 @@ int run_batch(psdm_engine* e, const BatchJob& j, int max_slots) {
         }
     }
     int next = 0;
+    if (rc == PSDM_OK && regions_on(e) && e->ckpt_interval == 0) {
+        rc = run_batch_regions(e, j, slots, &next);  // the others as one work list, below
+    }
     for (int k = 0; rc == PSDM_OK && k < nslots && next < j.nshots; ++k) rc = batch_start(e, j, slots[k], next++);
     // Run a slot's program up to its next launch; a finished shot hands over
     // its image and the slot takes the next shot.

@@ -285,6 +285,9 @@ int launch_step(int mode, const StepArgs& a, void* stream);
 // Quantize one snapshot outside a step launch (see StepArgs::q_*).
 int launch_quantize(const float* src, const unsigned int* amax, void* dst, float* iscale, int n, int kind16,
                     void* stream);
+// The same for `count` snapshots, each array advancing by its own stride (n).
+int launch_quantize_many(const float* src, const unsigned int* amax, void* dst, float* iscale, int n, int kind16,
+                         int count, void* stream);
 // Trace conditioning (rtm_condition.cu): Data_target (nt_taper per trace)
 // from Field_Data (nt_data per trace); w = taper weights (N_taper).
 struct CondArgs {
@@ -443,11 +446,12 @@ struct RegBlock {
     int soff;       // corners: its first column within the corner
     int pub0, npub, rcv0, nrcv, rcv_first;
 };
-// A region's share of one pass's geometry: its job, injection points
-// (RegParams::inj: offset in the region's source buffer, trace), the slots of
-// the row quads that hold them, and receivers (RegParams::rec: trace, shared offset).
+// A region's share of one pass's geometry: its job and number in the job's
+// plan, injection points (RegParams::inj: offset in the region's source
+// buffer, trace), the slots of the row quads that hold them, and receivers
+// (RegParams::rec: trace, shared offset).
 struct RegLoad {
-    int job, slot0, nslot, inj0, ninj, rec0, nrec, pad_;
+    int job, region, slot0, nslot, inj0, ninj, rec0, nrec;
 };
 // Values of one step.
 struct RegVar {
@@ -460,28 +464,27 @@ struct RegVar {
     int rec_t;         // receiver sample taken from level n at the start of this step, or -1
 };
 static_assert(sizeof(RegVar) % 8 == 0 && sizeof(RegVar) <= 128, "a warp fetches a RegVar");
-struct RegJob {
-    StepArgs a;         // arguments of the pass's first step
-    const RegVar* var;  // [nsteps]
-    void* board;        // 2 planes of npk 16-byte packets
-    int nsteps, npk;
-    unsigned int epoch; // tag of step i = epoch + i, used by no earlier launch on this board
-    int pad_;
-};
 struct RegPair {
     int x, y;
 };
-struct RegParams {
-    RegJob job;             // the only job, or
-    const RegJob* jobs;     // several jobs (RegLoad::job); null for one
-    const RegBlock* blocks;
-    const RegLoad* loads;   // by block
+// One pass of one shot, or some of its steps.
+struct RegJob {
+    StepArgs a;             // arguments of its first step
+    const RegVar* var;      // [nsteps]
+    const RegBlock* blocks; // its plan
     const RegPair* pub;     // packets published: index, shared offset | kRegSlow
     const int* rcv;         // packets received: shared offset | kRegSlow
+    void* board;            // 2 planes of npk 16-byte packets
+    int nsteps, npk;
+};
+struct RegParams {
+    RegJob job[kMaxSlots];  // the arithmetic's constants are those of job[0] for all
+    const RegLoad* loads;   // by block
     const signed char* slots;
     const RegPair* inj;
     const RegPair* rec;
     int* abort;             // device word, zero at launch
+    unsigned int epoch;     // tag of step i = epoch + i, used by no earlier launch on the boards
     float neg0;             // -0: keeps packed products apart from the sums that take them
 };
 struct RegPlan {
@@ -499,8 +502,12 @@ struct RegLists {
     size_t floats = 0, floats_img = 0;  // shared floats with the source buffers, and with the image
 };
 // Regions and packets of a padded grid for at most max_regions blocks of
-// max_floats shared floats.  False if the grid does not fit.
-bool plan_regions(const Grid& g, int fs, int max_regions, size_t max_floats, RegPlan* plan);
+// max_floats shared floats, with columns of `pitch` (0: the cheaper one).
+// False if the grid does not fit.
+bool plan_regions(const Grid& g, int fs, int max_regions, size_t max_floats, RegPlan* plan, int pitch = 0);
+// The estimated cycles of a step of that plan, without the plan; < 0 if the
+// grid does not fit.
+double region_step_cost(const Grid& g, int fs, int max_regions, size_t max_floats);
 // The regions' shares of a pass: injection points (linear cells x * ldz +
 // device row of interior cells, with their trace) and receivers.  False if
 // the source buffers do not fit.

@@ -262,14 +262,14 @@ struct Mail {
     uint4 v;
     bool asked;
 
-    __device__ __forceinline__ void init(const RegParams& rp, const RegBlock& b, const RegJob& job, int tid) {
+    __device__ __forceinline__ void init(const RegBlock& b, const RegJob& job, int tid) {
         board = static_cast<uint4*>(job.board);
         npk = job.npk;
         npub = b.npub;
         nrcv = b.nrcv;
         rcv_first = b.rcv_first;
-        pub = rp.pub + b.pub0;
-        rcv = rp.rcv + b.rcv0;
+        pub = job.pub + b.pub0;
+        rcv = job.rcv + b.rcv0;
         p0 = tid < npub ? pub[tid] : RegPair{0, 0};
         p1 = tid + kT < npub ? pub[tid + kT] : RegPair{0, 0};
         r0 = tid < nrcv ? rcv[tid] : 0;
@@ -434,7 +434,7 @@ template <int MODE, bool IMG, bool SPECIAL, int P>
 __device__ __forceinline__ bool run_interior(const RegParams& rp, const RegJob& job, RegShared& sh, const Consts& kc) {
     constexpr int P4 = P / 4, Q4 = (P - 8) / 4;
     constexpr int kAhead = MODE == 1 ? 2 : 1;  // columns of snapshot values in flight
-    const StepArgs& a = rp.job.a;
+    const StepArgs& a = rp.job[0].a;
     const RegBlock& b = sh.b;
     const int tid = threadIdx.x, nsteps = job.nsteps, np = sh.m.np, nslot = sh.ld.nslot, ninj = sh.ld.ninj,
               nrec = sh.ld.nrec, ldf = job.a.ldf, items = b.items, nbound = b.nbound, C = b.C, nqi = b.qb - b.qa;
@@ -450,7 +450,7 @@ __device__ __forceinline__ bool run_interior(const RegParams& rp, const RegJob& 
     em.comp = job.a.comp;
     em.isc = 1.f;
     Mail<P, false> mail;
-    mail.init(rp, b, job, tid);
+    mail.init(b, job, tid);
     // this thread's first boundary quad
     int bq = 0, bs = 0;
     if (tid < nbound) boundary_quad(b, tid, bq, bs);
@@ -540,7 +540,7 @@ __device__ __forceinline__ bool run_interior(const RegParams& rp, const RegJob& 
         // ---- the ring of level n
         bool ok = true;
         if (i > 0)
-            ok = mail.receive(g_smem + cur * np, nullptr, cur ^ 1, job.epoch + (unsigned int)i - 1u, rp.abort, tid);
+            ok = mail.receive(g_smem + cur * np, nullptr, cur ^ 1, rp.epoch + (unsigned int)i - 1u, rp.abort, tid);
         if (__syncthreads_or(!ok)) return false;
         // ---- boundary cells
         for (int j = tid; j < nbound; j += kT) {
@@ -580,7 +580,7 @@ __device__ __forceinline__ bool run_interior(const RegParams& rp, const RegJob& 
             sh.amax = 0u;
         }
         // ---- level n+1's edges to the neighbours
-        if (more) mail.send(g_smem + (cur ^ 1) * np, nullptr, cur, job.epoch + (unsigned int)i, tid);
+        if (more) mail.send(g_smem + (cur ^ 1) * np, nullptr, cur, rp.epoch + (unsigned int)i, tid);
     }
     return true;
 }
@@ -655,7 +655,7 @@ __device__ __forceinline__ void strip_update(const Consts& kc, const float2 (&k1
 template <int MODE, int P>
 __device__ __forceinline__ bool run_strip(const RegParams& rp, const RegJob& job, RegShared& sh, const Consts& kc) {
     constexpr int P4 = P / 4, Q4 = (P - 8) / 4;
-    const StepArgs& a = rp.job.a;
+    const StepArgs& a = rp.job[0].a;
     const RegBlock& b = sh.b;
     const int tid = threadIdx.x, nsteps = job.nsteps, np = sh.m.np, nq = sh.m.nq, ns = b.ns, nrec = sh.ld.nrec,
               items = b.items, nbound = b.nbound, C = b.C, nqi = b.qb - b.qa;
@@ -669,7 +669,7 @@ __device__ __forceinline__ bool run_strip(const RegParams& rp, const RegJob& job
     u.A = g_smem + sh.m.A;
     u.B = g_smem + sh.m.B;
     Mail<P, false> mail;
-    mail.init(rp, b, job, tid);
+    mail.init(b, job, tid);
     int bq = 0, bs = 0;
     if (tid < nbound) boundary_quad(b, tid, bq, bs);
     for (int i = 0; i < nsteps; ++i) {
@@ -719,7 +719,7 @@ __device__ __forceinline__ bool run_strip(const RegParams& rp, const RegJob& job
         // ---- the ring of level n
         bool ok = true;
         if (i > 0)
-            ok = mail.receive(g_smem + cur * np, nullptr, cur ^ 1, job.epoch + (unsigned int)i - 1u, rp.abort, tid);
+            ok = mail.receive(g_smem + cur * np, nullptr, cur ^ 1, rp.epoch + (unsigned int)i - 1u, rp.abort, tid);
         if (__syncthreads_or(!ok)) return false;
         // ---- boundary quads: stencil centres clamped at the grid's edge (p) and at both edges of the strip (phi)
         for (int j = tid; j < nbound; j += kT) {
@@ -740,7 +740,7 @@ __device__ __forceinline__ bool run_strip(const RegParams& rp, const RegJob& job
         if (more && nrec > 0) store_var(&sh.v[cur ^ 1], vnext, tid);
         __syncthreads();
         // ---- level n+1's edges to the neighbours
-        if (more) mail.send(g_smem + (cur ^ 1) * np, nullptr, cur, job.epoch + (unsigned int)i, tid);
+        if (more) mail.send(g_smem + (cur ^ 1) * np, nullptr, cur, rp.epoch + (unsigned int)i, tid);
     }
     return true;
 }
@@ -807,7 +807,7 @@ __device__ __forceinline__ void corner_cell(const StepArgs& a, const CornerStep&
 // All steps of a corner region, in run_interior's phases, one cell an item.
 template <int MODE, int P>
 __device__ __forceinline__ bool run_corner(const RegParams& rp, const RegJob& job, RegShared& sh) {
-    const StepArgs& a = rp.job.a;
+    const StepArgs& a = rp.job[0].a;
     const RegBlock& b = sh.b;
     const int tid = threadIdx.x, nsteps = job.nsteps, np = sh.m.np, nq = sh.m.nq, nphi = sh.m.nphi, nrec = sh.ld.nrec,
               items = b.items, nbound = b.nbound, fa = b.fa, fn = b.fb - fa, sa = b.sa, sn = b.sb - sa;
@@ -823,7 +823,7 @@ __device__ __forceinline__ bool run_corner(const RegParams& rp, const RegJob& jo
     u.A = g_smem + sh.m.A;
     u.B = g_smem + sh.m.B;
     Mail<P, true> mail;
-    mail.init(rp, b, job, tid);
+    mail.init(b, job, tid);
     for (int i = 0; i < nsteps; ++i) {
         const int cur = i & 1;
         const bool more = i + 1 < nsteps;
@@ -845,7 +845,7 @@ __device__ __forceinline__ bool run_corner(const RegParams& rp, const RegJob& jo
         bool ok = true;
         if (i > 0)
             ok = mail.receive(g_smem + cur * np, g_smem + sh.m.phi + cur * nphi, cur ^ 1,
-                              job.epoch + (unsigned int)i - 1u, rp.abort, tid);
+                              rp.epoch + (unsigned int)i - 1u, rp.abort, tid);
         if (__syncthreads_or(!ok)) return false;
         // rows outside [fa, fb) of every column, then the other rows of the columns outside [sa, sb)
 #pragma unroll 1
@@ -864,7 +864,7 @@ __device__ __forceinline__ bool run_corner(const RegParams& rp, const RegJob& jo
         }
         if (more && nrec > 0) store_var(&sh.v[cur ^ 1], vnext, tid);
         __syncthreads();
-        if (more) mail.send(u.pn, u.phxo, cur, job.epoch + (unsigned int)i, tid);
+        if (more) mail.send(u.pn, u.phxo, cur, rp.epoch + (unsigned int)i, tid);
     }
     return true;
 }
@@ -886,16 +886,18 @@ __global__ void __launch_bounds__(kT, 1) region_kernel(const __grid_constant__ R
     constexpr int Q = P - 8;
     __shared__ __align__(16) RegShared sh;
     const int tid = threadIdx.x;
-    for (int w = tid; w < (int)(sizeof(RegBlock) / 4); w += kT)
-        reinterpret_cast<int*>(&sh.b)[w] = reinterpret_cast<const int*>(rp.blocks + blockIdx.x)[w];
     for (int w = tid; w < (int)(sizeof(RegLoad) / 4); w += kT)
         reinterpret_cast<int*>(&sh.ld)[w] = reinterpret_cast<const int*>(rp.loads + blockIdx.x)[w];
     if (tid == 0) sh.amax = 0u;
     __syncthreads();
     // The constants of the arithmetic (a) are those of every job; the job's
     // own pointers and sizes are ja's.
-    const StepArgs& a = rp.job.a;
-    const RegJob& job = rp.jobs != nullptr ? rp.jobs[sh.ld.job] : rp.job;
+    const StepArgs& a = rp.job[0].a;
+    const RegJob& job = rp.job[sh.ld.job];
+    if (job.nsteps <= 0) return;
+    for (int w = tid; w < (int)(sizeof(RegBlock) / 4); w += kT)
+        reinterpret_cast<int*>(&sh.b)[w] = reinterpret_cast<const int*>(job.blocks + sh.ld.region)[w];
+    __syncthreads();
     const StepArgs& ja = job.a;
     const RegBlock& b = sh.b;
     RegSmem& m = sh.m;
@@ -1140,15 +1142,15 @@ int cut_part(Part* p, int P, double target, size_t max_floats, int budget) {
     return best;
 }
 
-}  // namespace
-
-bool plan_regions(const Grid& g, int fs, int max_regions, size_t max_floats, RegPlan* plan) {
-    *plan = RegPlan{};
+// The parts of a padded grid; false if a region of it could be narrower than
+// a packet.
+bool grid_parts(const Grid& g, int fs, int max_regions, std::vector<Part>* out) {
     // packets carry 3 cells of one region, so every region is 3 cells wide;
     // strips are at least 8
     if (g.ny < 3 || g.nx < 3 || g.dn < 8 || max_regions < 1) return false;
     const int dn = g.dn, d0 = dn + g.zoff, zb = d0 + g.ny, xr = dn + g.nx;
-    std::vector<Part> parts;
+    std::vector<Part>& parts = *out;
+    parts.clear();
     parts.push_back({kRegInterior, 0, 0, 0, d0, dn, g.ny, g.nx});
     parts.push_back({kRegStrip, 0, 1, 0, d0, 0, g.ny, dn});
     parts.push_back({kRegStrip, 0, 0, 0, d0, xr, g.ny, dn});
@@ -1160,26 +1162,54 @@ bool plan_regions(const Grid& g, int fs, int max_regions, size_t max_floats, Reg
         parts.push_back({kRegCorner, 0, 1, 1, g.zoff, 0, dn, dn});
         parts.push_back({kRegCorner, 0, 0, 1, g.zoff, xr, dn, dn});
     }
-    // The pitch with the cheaper step.
-    double best = 1e30;
-    for (int P : kRegPitches) {
-        auto total = [&](double target) {
-            int n = 0;
-            for (Part& p : parts) {
-                const int k = cut_part(&p, P, target, max_floats, max_regions);
-                if (k == 0) return 1 << 20;
-                n += k;
-            }
-            return n;
-        };
-        double lo = 0, hi = 1e7;
-        if (total(hi) > max_regions) continue;
-        for (int it = 0; it < 30 && hi - lo > 10; ++it) {
-            const double mid = it < 8 ? std::sqrt(std::max(lo, 100.0) * hi) : 0.5 * (lo + hi);
-            (total(mid) <= max_regions ? hi : lo) = mid;
+    return true;
+}
+
+// The cheapest largest region of the parts with columns of P; < 0 if they do
+// not fit.
+double cheapest_cut(std::vector<Part>& parts, int P, int max_regions, size_t max_floats) {
+    auto total = [&](double target) {
+        int n = 0;
+        for (Part& p : parts) {
+            const int k = cut_part(&p, P, target, max_floats, max_regions);
+            if (k == 0) return 1 << 20;
+            n += k;
         }
-        if (hi < best) {
-            best = hi;
+        return n;
+    };
+    double lo = 0, hi = 1e7;
+    if (total(hi) > max_regions) return -1.0;
+    for (int it = 0; it < 30 && hi - lo > 10; ++it) {
+        const double mid = it < 8 ? std::sqrt(std::max(lo, 100.0) * hi) : 0.5 * (lo + hi);
+        (total(mid) <= max_regions ? hi : lo) = mid;
+    }
+    return hi;
+}
+
+}  // namespace
+
+double region_step_cost(const Grid& g, int fs, int max_regions, size_t max_floats) {
+    std::vector<Part> parts;
+    if (!grid_parts(g, fs, max_regions, &parts)) return -1.0;
+    double best = -1.0;
+    for (int P : kRegPitches) {
+        const double c = cheapest_cut(parts, P, max_regions, max_floats);
+        if (c >= 0 && (best < 0 || c < best)) best = c;
+    }
+    return best;
+}
+
+bool plan_regions(const Grid& g, int fs, int max_regions, size_t max_floats, RegPlan* plan, int pitch) {
+    *plan = RegPlan{};
+    std::vector<Part> parts;
+    if (!grid_parts(g, fs, max_regions, &parts)) return false;
+    const int dn = g.dn, d0 = dn + g.zoff;
+    double best = -1.0;
+    for (int P : kRegPitches) {
+        if (pitch != 0 && P != pitch) continue;
+        const double c = cheapest_cut(parts, P, max_regions, max_floats);
+        if (c >= 0 && (best < 0 || c < best)) {
+            best = c;
             plan->pitch = P;
         }
     }
@@ -1303,6 +1333,7 @@ bool region_loads(const RegPlan& plan, const Grid& g, size_t max_floats, int nin
     for (int id = 0; id < n; ++id) {
         const RegBlock& r = plan.blocks[id];
         RegLoad& l = out->loads[id];
+        l.region = id;
         l.slot0 = (int)out->slots.size();
         std::vector<signed char> slot(quads(r.nf), -1);
         l.inj0 = (int)out->inj.size();

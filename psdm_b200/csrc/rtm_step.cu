@@ -1210,6 +1210,22 @@ int launch_quantize(const float* src, const unsigned int* amax, void* dst, float
     return (int)cudaGetLastError();
 }
 
+// A snapshot a grid row: the region form stages many before they are converted.
+__global__ void quantize_many_kernel(const float* src, const unsigned int* amax, unsigned short* dst, float* iscale,
+                                     int n, int kind16) {
+    const size_t m = blockIdx.y;
+    quantize_part(src + m * n, amax + m, dst + m * n, iscale + m, n, kind16, threadIdx.y * 32 + threadIdx.x);
+}
+
+int launch_quantize_many(const float* src, const unsigned int* amax, void* dst, float* iscale, int n, int kind16,
+                         int count, void* stream) {
+    if (n <= 0 || count <= 0) return 0;
+    const dim3 grid(min((n / 4 + NT - 1) / NT, 148), count);
+    quantize_many_kernel<<<grid, dim3(32, NWARP), 0, (cudaStream_t)stream>>>(
+        src, amax, static_cast<unsigned short*>(dst), iscale, n, kind16);
+    return (int)cudaGetLastError();
+}
+
 template <int FIXED>
 int launch_batch(const BatchParams& bp, int num_sms, cudaStream_t stream) {
     const int total = bp.first[bp.nslots];

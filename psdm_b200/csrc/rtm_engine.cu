@@ -127,6 +127,16 @@ struct psdm_engine {
     std::map<int, cudaGraphExec_t> bgraphs;  // batched launches: an executable graph per run length
     bool recon = false;     // FP32 shots reconstruct the source wavefield from a saved band
     std::map<std::pair<int, int>, std::array<int, 2>> fft_plans;  // (length, batch) -> cuFFT plans
+    // Designed filters (twiddles and response on the device) by length, step,
+    // type and band; the oldest gives way.
+    struct Filter {
+        int nt = 0, typef = 0;
+        float dt = 0.f, f1 = 0.f, f2 = 0.f;
+        void *tw = nullptr, *G = nullptr;
+    };
+    static constexpr int kFilters = 4;
+    Filter filters[kFilters];
+    int filter_next = 0;
     // dt -> (fast division exact, 1/dt, lo, hi); the check costs ~50 ms
     std::map<float, std::pair<int, std::vector<float>>> div_cache;
 
@@ -181,6 +191,7 @@ struct psdm_engine {
         reg_board = nullptr;
         for (auto& kv : fft_plans) destroy_fft_plans(kv.second.data());
         fft_plans.clear();
+        for (Filter& f : filters) f = Filter{};
         for (auto& kv : bufs)
             if (kv.second.ptr) CUDA_TRY(cudaFree(kv.second.ptr));
         bufs.clear();
@@ -3305,22 +3316,22 @@ int psdm_condition_traces_device(psdm_engine* e, const psdm_conditioning* c, int
         return fail(PSDM_ERR_ARG, "inconsistent trace lengths");
     if (dt_data != dt_prop && (dt_data <= 0.f || dt_prop <= 0.f)) return fail(PSDM_ERR_ARG, "time steps must be > 0");
     if (NumRec == 0) return PSDM_OK;
-    int *d_cut = nullptr, *d_sf = nullptr;
-    float* d_w = nullptr;
-    TRY(e->get("cond_cut", (size_t)NumRec, &d_cut));
-    TRY(e->get("cond_sf", (size_t)NumRec, &d_sf));
-    TRY(e->get("cond_w", (size_t)N_taper, &d_w));
-    std::vector<float> w(N_taper);
-    for (int n = 0; n < N_taper; ++n) w[n] = taper_weight(n, N_taper);
-    CUDA_TRY(cudaMemcpyAsync(d_cut, nt_cut, NumRec * sizeof(int), cudaMemcpyHostToDevice, e->stream));
-    CUDA_TRY(cudaMemcpyAsync(d_sf, nt_sf, NumRec * sizeof(int), cudaMemcpyHostToDevice, e->stream));
-    CUDA_TRY(cudaMemcpyAsync(d_w, w.data(), N_taper * sizeof(float), cudaMemcpyHostToDevice, e->stream));
+    // cuts, sea-floor samples and taper weights in one upload
+    static_assert(sizeof(int) == sizeof(float), "the lists share a buffer");
+    const size_t words = 2 * (size_t)NumRec + N_taper;
+    float* d_list = nullptr;
+    TRY(e->get("cond_list", words, &d_list));
+    std::vector<float> list(words);
+    std::memcpy(list.data(), nt_cut, NumRec * sizeof(int));
+    std::memcpy(list.data() + NumRec, nt_sf, NumRec * sizeof(int));
+    for (int n = 0; n < N_taper; ++n) list[2 * (size_t)NumRec + n] = taper_weight(n, N_taper);
+    CUDA_TRY(cudaMemcpyAsync(d_list, list.data(), words * sizeof(float), cudaMemcpyHostToDevice, e->stream));
     CondArgs a;
     a.field = d_Field_Data;
     a.out = d_Data_target;
-    a.nt_cut = d_cut;
-    a.nt_sf = d_sf;
-    a.w = d_w;
+    a.nt_cut = reinterpret_cast<const int*>(d_list);
+    a.nt_sf = reinterpret_cast<const int*>(d_list) + NumRec;
+    a.w = d_list + 2 * (size_t)NumRec;
     a.nrec = NumRec;
     a.nt_data = nt_data;
     a.nt_prop2 = nt_prop2;
@@ -3355,12 +3366,57 @@ int psdm_condition_traces(psdm_engine* e, const psdm_conditioning* c, int32_t Nu
     return sync(e);
 }
 
+// The filter of traces of nt samples, designed on first use (M points: see
+// design_filter).
+static int designed_filter(psdm_engine* e, int nt, float dt, int typef, float f1, float f2, int M,
+                           const psdm_engine::Filter** out) {
+    for (const auto& f : e->filters)
+        if (f.nt == nt && f.typef == typef && f.dt == dt && f.f1 == f1 && f.f2 == f2) {
+            *out = &f;
+            return PSDM_OK;
+        }
+    const int k = e->filter_next, ts = 24 * nt;  // zero_pad = 24 (auxiliar.f90:511-512)
+    e->filter_next = (k + 1) % psdm_engine::kFilters;
+    psdm_engine::Filter& f = e->filters[k];
+    f = psdm_engine::Filter{};
+    const std::string t = std::to_string(k);
+    float *tw = nullptr, *G = nullptr;
+    char* work = nullptr;
+    const size_t hb = (size_t)(ts / 2 + 1) * sizeof(std::complex<double>);
+    TRY(e->get(("filt_tw" + t).c_str(), (size_t)4 * M, &tw));
+    TRY(e->get(("filt_G" + t).c_str(), (size_t)2 * (M + 1), &G));
+    TRY(e->get("filt_design", filter_design_bytes(ts, nt, M), &work));
+    std::vector<std::complex<double>> H(ts / 2 + 1);
+    butterworth_response_f64(ts, 1.f / dt, typef, f1, f2, H.data());
+    CUDA_TRY(cudaMemcpyAsync(work, H.data(), hb, cudaMemcpyHostToDevice, e->stream));
+    const int rc = design_filter(work, work + hb, ts, nt, M, tw, G, e->stream);
+    if (rc) return fail(PSDM_ERR_CUDA, "filter design launch: %s", cudaGetErrorString((cudaError_t)rc));
+    e->launches += 5;
+    f.nt = nt;
+    f.typef = typef;
+    f.dt = dt;
+    f.f1 = f1;
+    f.f2 = f2;
+    f.tw = tw;
+    f.G = G;
+    *out = &f;
+    return PSDM_OK;
+}
+
 int psdm_freq_filter_device(psdm_engine* e, float* d_traces, int32_t nt, float dt, int32_t Num, int32_t typef,
                             float f1, float f2) {
     TRY(check_engine(e));
     if (!d_traces || nt < 1 || Num < 0 || !(dt > 0.f)) return fail(PSDM_ERR_ARG, "null argument or empty trace");
     if (typef < 1 || typef > 3) return fail(PSDM_ERR_ARG, "typef must be 1 (low-pass), 2 (high-pass) or 3 (band-pass)");
     if (Num == 0) return PSDM_OK;
+    if (const int M = filter_points(nt)) {
+        const psdm_engine::Filter* f = nullptr;
+        TRY(designed_filter(e, nt, dt, typef, f1, f2, M, &f));
+        const int rc = launch_filter(d_traces, nt, Num, M, f->tw, f->G, e->stream);
+        if (rc) return fail(PSDM_ERR_CUDA, "frequency filter launch: %s", cudaGetErrorString((cudaError_t)rc));
+        e->launches += 1;
+        return PSDM_OK;
+    }
     const int ts = 24 * nt;  // zero_pad = 24 (auxiliar.f90:511-512)
     std::vector<std::complex<float>> H(ts);
     butterworth_response(ts, 1.f / dt, typef, f1, f2, H.data());

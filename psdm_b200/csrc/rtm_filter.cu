@@ -4,9 +4,20 @@
 // placed at the end of a zero buffer 24 times its length, transformed,
 // multiplied by the response (and by 1/n, the forward scaling of the
 // reference's FFT), transformed back, and the real part of the last nt
-// samples is kept; see filter_traces for the half-spectrum form used here.  The transforms are cuFFT's (a library FFT, like the
-// reference's vendored FFTPACK); the results agree with the reference's
-// arithmetic to FP32 rounding, not bit for bit.
+// samples is kept.
+//
+// Only lags below nt of that circular convolution reach the samples that are
+// kept, so a transform of N >= 2 nt - 1 points (a power of two) with the
+// response's impulse response cut to those lags gives the same samples with
+// a twelfth of the work.  filter_kernel does it in one pass, a block a trace:
+// real transform, response and inverse in shared memory, so that a trace is
+// read and written once.  480 traces of 2004 samples: 18.6 us, against 1.41 ms
+// with batched cuFFT transforms of the padded traces (three passes over 92 MB
+// buffers); the error against 64 bits is the same 9.5e-5, that of the
+// reference's single-precision frequency sums.
+// Traces of more than 16384 samples, whose transform does not fit a block's
+// shared memory, take the cuFFT form (filter_traces).  The results agree
+// with the reference's arithmetic to FP32 rounding, not bit for bit.
 
 #include <cuda_runtime.h>
 #include <cuComplex.h>
@@ -98,6 +109,267 @@ size_t filter_work_floats(int ts, int num) {
     const size_t real = ((size_t)ts * num + 3) & ~(size_t)3;  // complex half starts 16-byte aligned
     return real + (size_t)(ts / 2 + 1) * num * 2;
 }
+
+// ---- the one-pass form
+
+namespace {
+
+__device__ __forceinline__ float2 cmul(const float2& a, const float2& b) {
+    return make_float2(fmaf(a.x, b.x, -__fmul_rn(a.y, b.y)), fmaf(a.x, b.y, __fmul_rn(a.y, b.x)));
+}
+__device__ __forceinline__ float2 cadd(const float2& a, const float2& b) { return make_float2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float2 csub(const float2& a, const float2& b) { return make_float2(a.x - b.x, a.y - b.y); }
+// a times -i (forward) or i (inverse)
+template <bool INV>
+__device__ __forceinline__ float2 rot(const float2& a) {
+    return INV ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
+}
+template <bool INV>
+__device__ __forceinline__ void dft4(float2& a, float2& b, float2& c, float2& d) {
+    const float2 s = cadd(a, c), t = csub(a, c), u = cadd(b, d), v = rot<INV>(csub(b, d));
+    a = cadd(s, u);
+    b = cadd(t, v);
+    c = csub(s, u);
+    d = csub(t, v);
+}
+template <bool INV, int R>
+__device__ __forceinline__ void dft(float2 (&v)[R]) {
+    if (R == 2) {
+        const float2 t = v[0];
+        v[0] = cadd(t, v[1]);
+        v[1] = csub(t, v[1]);
+    } else if (R == 4) {
+        dft4<INV>(v[0], v[1], v[2], v[3]);
+    } else {
+        float2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+        dft4<INV>(e[0], e[1], e[2], e[3]);
+        dft4<INV>(o[0], o[1], o[2], o[3]);
+        const float r = 0.70710678118654752f;
+        o[1] = cmul(o[1], make_float2(r, INV ? r : -r));
+        o[2] = rot<INV>(o[2]);
+        o[3] = cmul(o[3], make_float2(-r, INV ? r : -r));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            v[k] = cadd(e[k], o[k]);
+            v[k + 4] = csub(e[k], o[k]);
+        }
+    }
+}
+
+// Shared index of point i: a pad after every 16 points keeps the strided
+// stores of the first stages off one bank.
+__device__ __forceinline__ int padded(int i) { return i + (i >> 4); }
+
+// One self-sorting stage of radix R over M points held E a thread: butterfly
+// b = s p + q takes points b + k M / R and leaves q + s (R p + k), times
+// W_M^(s p k) (tw: W_2M).
+template <bool INV, int R, int E>
+__device__ __forceinline__ void fft_stage(float2* z, const float2* __restrict__ tw, int M, int ls, int tid, int T) {
+    constexpr int B = E / R;
+    const int nb = M / R;
+    float2 v[B][R];
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+        const int b = tid + u * T;
+        if (b >= nb) break;
+#pragma unroll
+        for (int k = 0; k < R; ++k) v[u][k] = z[padded(b + k * nb)];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+        const int b = tid + u * T;
+        if (b >= nb) break;
+        const int p = b >> ls, q = b & ((1 << ls) - 1);
+        dft<INV, R>(v[u]);
+        z[padded(q + ((R * p) << ls))] = v[u][0];
+#pragma unroll
+        for (int k = 1; k < R; ++k) {
+            float2 w = __ldg(tw + (((p * k) << ls) << 1));
+            if (INV) w.y = -w.y;
+            z[padded(q + ((R * p + k) << ls))] = cmul(v[u][k], w);
+        }
+    }
+    __syncthreads();
+}
+
+template <bool INV, int E>
+__device__ __forceinline__ void fft(float2* z, const float2* tw, int M, int logM, int tid, int T) {
+    int ls = 0;
+    for (; logM - ls >= 3; ls += 3) fft_stage<INV, 8, E>(z, tw, M, ls, tid, T);
+    if (logM - ls == 2) fft_stage<INV, 4, E>(z, tw, M, ls, tid, T);
+    if (logM - ls == 1) fft_stage<INV, 2, E>(z, tw, M, ls, tid, T);
+}
+
+// One trace a block: y = x * h on a circle of 2M points.  The real trace is
+// transformed as M complex points (even samples + i odd samples); X(k) and
+// X(M - k) are separated, multiplied by the response G (M + 1 bins, 1/M
+// included) and put together again.  A trace of zeros is left as it is
+// (is_not_cero).
+template <int E>
+__global__ void __launch_bounds__(1024) filter_kernel(float* tr, int nt, int M, int logM, const float2* __restrict__ tw,
+                              const float2* __restrict__ G) {
+    extern __shared__ float2 z[];
+    const int tid = threadIdx.x, T = blockDim.x;
+    float* x = tr + (size_t)blockIdx.x * nt;
+    int any = 0;
+    for (int n = tid; n < M; n += T) {
+        const float a = 2 * n < nt ? x[2 * n] : 0.f, b = 2 * n + 1 < nt ? x[2 * n + 1] : 0.f;
+        z[padded(n)] = make_float2(a, b);
+        any |= a != 0.f || b != 0.f;
+    }
+    if (!__syncthreads_or(any)) return;
+    fft<false, E>(z, tw, M, logM, tid, T);
+    for (int k = tid; k <= M / 2; k += T) {
+        const int m = (M - k) & (M - 1);
+        const float2 a = z[padded(k)], c = z[padded(m)], w = __ldg(tw + k);
+        const float2 e = make_float2(0.5f * (a.x + c.x), 0.5f * (a.y - c.y));
+        const float2 o = make_float2(0.5f * (a.y + c.y), -0.5f * (a.x - c.x));  // (a - conj c) / 2i
+        const float2 wo = cmul(w, o);
+        const float2 gm = __ldg(G + M - k);
+        const float2 y = cmul(cadd(e, wo), __ldg(G + k));
+        const float2 ym = cmul(csub(e, wo), make_float2(gm.x, -gm.y));  // conj of Y(M - k)
+        const float2 e2 = make_float2(0.5f * (y.x + ym.x), 0.5f * (y.y + ym.y));
+        const float2 o2 = cmul(make_float2(0.5f * (y.x - ym.x), 0.5f * (y.y - ym.y)), make_float2(w.x, -w.y));
+        z[padded(k)] = make_float2(e2.x - o2.y, e2.y + o2.x);  // e2 + i o2
+        if (m != k) z[padded(m)] = make_float2(e2.x + o2.y, o2.x - e2.y);  // conj e2 + i conj o2
+    }
+    __syncthreads();
+    fft<true, E>(z, tw, M, logM, tid, T);
+    for (int n = tid; n < nt; n += T) {
+        const float2 v = z[padded(n >> 1)];
+        x[n] = (n & 1) ? v.y : v.x;
+    }
+}
+
+// exp(2 pi i j / n), j < n
+__global__ void roots_kernel(double2* w, int n) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= n) return;
+    double s, c;
+    sincospi(2.0 * j / n, &s, &c);
+    w[j] = make_double2(c, s);
+}
+
+// Sum of a block's doubles in its first thread.
+__device__ double block_sum(double v) {
+    __shared__ double part[32];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double s = 0.0;
+    if (threadIdx.x == 0)
+        for (int k = 0; k < (int)(blockDim.x + 31) / 32; ++k) s += part[k];
+    return s;
+}
+
+// Impulse response at lag l = blockIdx.x - (nt - 1) of the response H (bins 0
+// .. ts/2) on a circle of ts points; of the last bin only the real part counts.
+__global__ void impulse_kernel(const double2* __restrict__ H, const double2* __restrict__ root, int ts, int nt,
+                               double* h) {
+    const int l = blockIdx.x - (nt - 1), half = ts / 2, step = (int)((long long)blockDim.x * (l < 0 ? l + ts : l) % ts);
+    long long at = (long long)threadIdx.x * (l < 0 ? l + ts : l) % ts;
+    double s = 0.0;
+    for (int k = threadIdx.x; k <= half; k += blockDim.x) {
+        const double2 w = root[at], g = H[k];
+        s += (k == 0 || k == half ? 1.0 : 2.0) * (g.x * w.x - (k == half ? 0.0 : g.y * w.y));
+        at += step;
+        if (at >= ts) at -= ts;
+    }
+    s = block_sum(s);
+    if (threadIdx.x == 0) h[blockIdx.x] = s / ts;
+}
+
+// Bin k = blockIdx.x of the impulse response's transform of N = 2M points, / M.
+__global__ void response_kernel(const double* __restrict__ h, const double2* __restrict__ root, int nt, int M, float2* G) {
+    const int N = 2 * M, k = blockIdx.x;
+    double re = 0.0, im = 0.0;
+    for (int i = threadIdx.x; i < 2 * nt - 1; i += blockDim.x) {
+        const double2 w = root[(int)((long long)k * ((i - (nt - 1) + N) % N) % N)];
+        re += h[i] * w.x;
+        im -= h[i] * w.y;
+    }
+    re = block_sum(re);
+    im = block_sum(im);
+    if (threadIdx.x == 0) G[k] = make_float2((float)(re / M), (float)(im / M));
+}
+
+// exp(-2 pi i j / n) in single precision
+__global__ void twiddle_kernel(const double2* __restrict__ root, float2* tw, int n) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < n) tw[j] = make_float2((float)root[j].x, (float)-root[j].y);
+}
+
+}  // namespace
+
+int filter_points(int nt) {
+    int M = 256;
+    while (2 * M < 2 * nt - 1) M *= 2;
+    return M <= kFilterMaxPoints ? M : 0;
+}
+
+void butterworth_response_f64(int ts, float fe, int typef, float f1, float fc, std::complex<double>* H) {
+    // butterworth_response's parameters and frequencies (its single-precision
+    // sums), the response itself in double: s is purely imaginary, s = i b
+    const int n = 6;
+    const float pi = 3.14159265f, fs = 40.f, f0 = std::sqrt(f1 * fc), Q = f0 / (fc - f1);
+    float f = 0.f;
+    for (int j = 0; j <= ts / 2; ++j) {
+        const double x = f;
+        const double b = typef == 1 ? x / fc : (typef == 2 ? -fs / x : (double)Q * (x / f0 - f0 / x));
+        std::complex<double> B(1.0, 0.0);
+        for (int k = 1; k <= n / 2; ++k) {
+            const double c = std::cos((float(2 * k + n - 1) * pi) / float(2 * n));
+            const double re = 1.0 - b * b, im = -2.0 * b * c;
+            B = std::complex<double>(B.real() * re - B.imag() * im, B.real() * im + B.imag() * re);
+        }
+        const double q = B.real() * B.real() + B.imag() * B.imag();
+        H[j] = std::complex<double>(B.real() / q, -B.imag() / q);
+        f = f + fe / float(ts);
+    }
+    H[0] = typef == 1 ? 1.0 : 0.0;
+}
+
+size_t filter_design_bytes(int ts, int nt, int M) {
+    return ((size_t)ts + 2 * M + ts / 2 + 1) * sizeof(double2) + (size_t)(2 * nt) * sizeof(double);
+}
+
+int design_filter(const void* d_H, void* work, int ts, int nt, int M, void* d_tw, void* d_G, void* stream) {
+    cudaStream_t st = (cudaStream_t)stream;
+    double2* root = static_cast<double2*>(work);
+    double2* rootN = root + ts;
+    double* h = reinterpret_cast<double*>(rootN + 2 * M);
+    roots_kernel<<<(ts + 255) / 256, 256, 0, st>>>(root, ts);
+    roots_kernel<<<(2 * M + 255) / 256, 256, 0, st>>>(rootN, 2 * M);
+    impulse_kernel<<<2 * nt - 1, 256, 0, st>>>(static_cast<const double2*>(d_H), root, ts, nt, h);
+    response_kernel<<<M + 1, 256, 0, st>>>(h, rootN, nt, M, static_cast<float2*>(d_G));
+    twiddle_kernel<<<(2 * M + 255) / 256, 256, 0, st>>>(rootN, static_cast<float2*>(d_tw), 2 * M);
+    return (int)cudaGetLastError();
+}
+
+template <int E>
+int launch_filter_t(float* d_tr, int nt, int num, int M, const void* d_tw, const void* d_G, cudaStream_t st) {
+    int logM = 0;
+    while ((1 << logM) < M) ++logM;
+    const size_t bytes = (size_t)(M + M / 16) * sizeof(float2);
+    if (bytes > 48 * 1024) {
+        const cudaError_t rc = cudaFuncSetAttribute(filter_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                    (int)bytes);
+        if (rc != cudaSuccess) return (int)rc;
+    }
+    filter_kernel<E><<<num, M / E, bytes, st>>>(d_tr, nt, M, logM, static_cast<const float2*>(d_tw),
+                                                static_cast<const float2*>(d_G));
+    return (int)cudaGetLastError();
+}
+
+int launch_filter(float* d_tr, int nt, int num, int M, const void* d_tw, const void* d_G, void* stream) {
+    // 8 points a thread up to 1024 threads
+    if (M <= 8192) return launch_filter_t<8>(d_tr, nt, num, M, d_tw, d_G, (cudaStream_t)stream);
+    return launch_filter_t<16>(d_tr, nt, num, M, d_tw, d_G, (cudaStream_t)stream);
+}
+
+// ---- the cuFFT form
 
 // The reference transforms the real trace as a complex one and keeps the real
 // part of the inverse.  The product of a real trace's spectrum with the

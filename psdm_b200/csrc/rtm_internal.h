@@ -304,8 +304,19 @@ int launch_condition(const CondArgs& c, void* stream);
 
 // Frequency filter (rtm_filter.cu): Butterworth response of length ts on the
 // host, and the filtering of num traces of nt samples in place on `stream`
-// with a batched length-ts cuFFT plan (an int handle stored at plan_ptr).
+// with batched length-ts cuFFT plans.
 void butterworth_response(int ts, float fe, int typef, float f1, float fc, std::complex<float>* H);
+// One-pass form (traces of up to 16384 samples): a transform of 2M points,
+// M = filter_points(nt) (0: too long).  A filter is designed once for its
+// length, step and band: twiddles (2M float2) and response (M + 1 float2)
+// from the response H (bins 0 .. ts/2, double2, at d_H) with `work` of
+// filter_design_bytes beside H.
+constexpr int kFilterMaxPoints = 16384;
+int filter_points(int nt);
+void butterworth_response_f64(int ts, float fe, int typef, float f1, float fc, std::complex<double>* H);
+size_t filter_design_bytes(int ts, int nt, int M);
+int design_filter(const void* d_H, void* work, int ts, int nt, int M, void* d_tw, void* d_G, void* stream);
+int launch_filter(float* d_tr, int nt, int num, int M, const void* d_tw, const void* d_G, void* stream);
 int make_fft_plans(int ts, int num, int* plans);  // plans[0] real-to-complex, plans[1] complex-to-real
 void destroy_fft_plans(int* plans);
 size_t filter_work_floats(int ts, int num);

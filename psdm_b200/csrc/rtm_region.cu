@@ -1117,13 +1117,15 @@ int piece_slow(int n, int k) { return (n + k - 1) / k; }
 int cut_part(Part* p, int P, double target, size_t max_floats, int budget) {
     const int nf = p->nfast(), ns = p->nslow();
     int best = 0;
-    // interior: both ways; strips: along the strip; corners: in columns
+    // interior: both ways; strips: along the strip; corners: in columns of at least
+    // 7, so that the clamped stencils at the grid's edge (columns 0 to 6) and of phi at the corner's
+    // inner edge lie in one region: those cells are updated before the ring arrives
     const int amax = p->type == kRegCorner ? 1 : std::max(1, std::min(quads(nf) / 2, budget));
     for (int ka = 1; ka <= amax; ++ka) {
         const int f = std::min(nf, piece_fast(nf, ka));
         if (f > P - 8) continue;
         const int bmax = p->type == kRegInterior ? std::max(1, std::min(ns / 3, budget / ka))
-                                                 : (p->type == kRegCorner ? std::max(1, std::min(ns / 6, budget)) : 1);
+                                                 : (p->type == kRegCorner ? std::max(1, std::min(ns / 7, budget)) : 1);
         auto good = [&](int kb) {
             const int s = piece_slow(ns, kb);
             return region_floats(P, p->type, f, s, 0, false) + 64 <= max_floats && region_cost(p->type, f, s) <= target;

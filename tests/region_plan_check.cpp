@@ -3,6 +3,7 @@
 // exactly once, ring cells that a packet exchange leaves wrong, regions over
 // the shared-memory limit, injection or receiver entries that name another
 // cell, packets received more than once.
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <map>
@@ -98,6 +99,23 @@ int main(int argc, char** argv) {
             for (int f = 0; f < r.nf; ++f) {
                 const bool in = r.soff + s >= 0 && r.soff + s < g.dn;
                 wrong_ring += phi[b][(size_t)(s + 3) * r.Q + f] != (in ? id(r.z0 + f, r.x0 + s) : 0.0);
+            }
+    }
+    // inner cells are updated before the ring arrives: their stencils, clamped at the grid's edge and (phi)
+    // at the strip's edges, end inside the region
+    auto inside = [](int c, int n) { return c - 3 >= 0 && c + 3 < n; };
+    auto clamp = [](int v, int lo, int hi) { return v < lo ? lo : v > hi ? hi : v; };
+    for (const RegBlock& r : plan.blocks) {
+        const bool corner = r.type == kRegCorner, strip = r.type == kRegStrip;
+        const int fa = corner ? r.fa : 4 * r.qa, fb = corner ? r.fb : 4 * r.qb;
+        for (int s = r.sa; s < r.sb; ++s)
+            for (int f = fa; f < fb; ++f) {
+                const int sg = s + (corner ? r.soff : 0);  // within the strip or corner
+                const int cs = corner ? (r.low ? std::max(sg, 3) : std::min(sg, g.dn - 4)) - r.soff : s;
+                const int cp = strip || corner ? clamp(sg, 3, g.dn - 4) - (corner ? r.soff : 0) : s;
+                const int cz = corner ? (r.lowf ? std::max(f, 3) : std::min(f, r.nf - 4)) : f;
+                const bool grid_top = !corner && f < 3 && fa == 0, grid_end = !corner && f + 3 >= r.nf && fb >= r.nf;
+                over += !inside(cs, r.ns) || !inside(cp, r.ns) || (!grid_top && !grid_end && !inside(cz, r.nf));
             }
     }
     // injection points on two rows (every other column) and receivers anywhere

@@ -1,7 +1,9 @@
 """The region form's planner on the CPU: psdm::plan_regions covers every live
 cell of the padded grid by exactly one region within the shared-memory limit,
 one exchange of its packets fills every ring cell that a neighbour owns (and
-leaves rows above a free surface and cells outside the grid at zero), and
+leaves rows above a free surface and cells outside the grid at zero), the
+stencils of the cells updated before the ring arrives end inside the region,
+and
 psdm::region_loads names each injection point and receiver in the region that
 owns it.  tests/region_plan_check.cpp is compiled against the built engine
 library and run here, without a GPU."""
@@ -42,6 +44,7 @@ FLOATS = 57500  # a B200 block's dynamic shared memory beside the kernel's own
     (1200, 1136, 50, 1, 148),
     (1199, 1137, 50, 0, 148),
     (1500, 1210, 40, 1, 148),
+    (200, 400, 12, 1, 148),    # corners cut to their narrowest columns
 ])
 def test_regions_cover_grid_and_exchange_rings(checker, ny, nx, dPML, fs, regions):
     r = subprocess.run([checker, *map(str, (ny, nx, dPML, fs, regions, FLOATS))], capture_output=True, text=True,

@@ -430,10 +430,7 @@ int launch_resident(int mode, const ResParams& rp, void* stream);
 // ---- region pass kernel (rtm_region.cu) -------------------------------------
 // One cooperative launch per pass (of one shot, or of several shots side by
 // side), one block per region of the padded grid.
-#ifndef PSDM_REGION_THREADS
-#define PSDM_REGION_THREADS 384
-#endif
-constexpr int kRegThreads = PSDM_REGION_THREADS;
+constexpr int kRegThreads = 384;
 constexpr int kRegPitches[2] = {72, 136};  // pitch of the shared columns: a region has at most pitch - 8 rows (fast)
 constexpr int kRegMaxQuads = 32;  // row quads of a region
 constexpr int kRegInterior = 0, kRegStrip = 1, kRegCorner = 2;
@@ -449,7 +446,7 @@ struct RegBlock {
     int nq;
     // Inner cells, whose stencils end inside the region: row quads [qa, qb) x
     // slow positions [sa, sb) (corners: fast positions [fa, fb)), in `items` items
-    // of C slow positions; the other quads or cells are the nbound boundary items.
+    // of C slow positions (0: single quads, cells); the other quads or cells are the nbound boundary items.
     int qa, qb, fa, fb, sa, sb, C, items, nbound;
     int nslot;      // slots of the source buffer (set per pass)
     int fsrow;      // fast position 0 is the free-surface row

@@ -29,11 +29,13 @@
 // part with at most one region per multiprocessor.
 //
 // Measured on the B200 (a shot, against one launch per step): 1200 x 1136
-// window, 8000 steps 90.8 ms against 164.5 (forward step 10.4 -> 5.1 us,
-// backward 9.4 -> 6.4); 200 x 249, 3000 steps 19.9 against 53.4; 331 x 321
-// with C-PML on all sides, 1501 steps 9.6 against 39.9; 36 x 64, 260 steps
-// 1.53 against 4.51.  12 warps of up to 168 registers: 16 warps spill the
-// column loops (model of the first window 24.3 against 19.5 ms).
+// window, 8000 steps 89.0 ms against 164.5 (forward step 10.4 -> 5.0 us,
+// backward 9.4 -> 6.2); 200 x 249, 3000 steps 13.0 against 53.4; 331 x 321
+// with C-PML on all sides, 1501 steps 6.4 against 39.9; 36 x 64, 260 steps
+// 1.22 against 4.51.  12 warps of up to 168 registers: 16 warps spill the
+// column loops (model of the first window 24.3 against 19.5 ms), and two
+// blocks a multiprocessor halve a region's cells but double its packets
+// (first window 125 ms).
 //
 // The arithmetic of every cell is the step kernels' in their order, so the
 // results are the same bit for bit; the pass starts from and leaves the same
@@ -427,7 +429,8 @@ __device__ __forceinline__ void boundary_quad(const RegBlock& b, int i, int& q, 
 
 // All steps of an interior region.  Inner cells (whose stencils do not touch
 // the ring) are updated while the ring's packets are on their way: a thread
-// slides down C columns of one row quad.  Then the ring, the boundary quads,
+// slides down C columns of one row quad, or takes single quads where that is
+// only one or two columns (C = 0).  Then the ring, the boundary quads,
 // and the packets of the new level.  SPECIAL: the region holds injection
 // points or the free surface.  Returns false when a wait gave up.
 template <int MODE, bool IMG, bool SPECIAL, int P>
@@ -482,8 +485,32 @@ __device__ __forceinline__ bool run_interior(const RegParams& rp, const RegJob& 
         const float4* src4 = reinterpret_cast<const float4*>(src + cur * nsrc);
         float amax_t = 0.f;
         mail.asked = false;
+        // one quad, all its operands from shared memory
+        auto single = [&](int q, int s, const Ahead& h) {
+            const float4* w = pc + s * P4 + 1 + q;
+            float4* po = pn + (s + 3) * P4 + 1 + q;
+            float4 win[7];
+#pragma unroll
+            for (int k = 0; k < 7; ++k) win[k] = w[k * P4];
+            const float4 pm = po[0];
+            float4 sv = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (SPECIAL && sh.slot[q] >= 0) sv = src4[sh.slot[q] * b.ns + s];
+            float4 out =
+                interior_update<SPECIAL>(kc, win, w[3 * P4 - 1], w[3 * P4 + 1], pm, c24[s * Q4 + q], sv);
+            if (zero_top && q == 0) out.x = 0.f;
+            emit_quad<MODE, IMG>(a, kc, em, out, pm, b.nf - 4 * q, b.f0 + s * ldf + 4 * q, img4 + s * Q4 + q, h,
+                                 amax_t);
+            po[0] = out;
+        };
         // ---- inner cells
-        for (int it = tid; it < items; it += kT) {
+        for (int j = tid; C == 0 && j < items; j += kT) {
+            const int col = j / nqi, q = b.qa + j - col * nqi, s = b.sa + col;
+            if (j + kT >= items) mail.request(cur ^ 1, tid, i > 0);
+            Ahead h;
+            if (MODE != 0 && em.field != nullptr) load_ahead<MODE, IMG>(em, b.f0 + s * ldf + 4 * q, h);
+            single(q, s, h);
+        }
+        for (int it = tid; C > 0 && it < items; it += kT) {
             const int ch = it / nqi, q = b.qa + it - ch * nqi, s0 = b.sa + ch * C, n = min(C, b.sb - s0);
             const float4* w = pc + s0 * P4 + 1 + q;
             float4* po = pn + (s0 + 3) * P4 + 1 + q;
@@ -549,20 +576,7 @@ __device__ __forceinline__ bool run_interior(const RegParams& rp, const RegJob& 
                 boundary_quad(b, j, q, s);
                 if (MODE != 0 && em.field != nullptr) load_ahead<MODE, IMG>(em, b.f0 + s * ldf + 4 * q, bh);
             }
-            const float4* w = pc + s * P4 + 1 + q;
-            float4* po = pn + (s + 3) * P4 + 1 + q;
-            float4 win[7];
-#pragma unroll
-            for (int k = 0; k < 7; ++k) win[k] = w[k * P4];
-            const float4 pm = po[0];
-            float4 sv = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (SPECIAL && sh.slot[q] >= 0) sv = src4[sh.slot[q] * b.ns + s];
-            float4 out =
-                interior_update<SPECIAL>(kc, win, w[3 * P4 - 1], w[3 * P4 + 1], pm, c24[s * Q4 + q], sv);
-            if (zero_top && q == 0) out.x = 0.f;
-            emit_quad<MODE, IMG>(a, kc, em, out, pm, b.nf - 4 * q, b.f0 + s * ldf + 4 * q, img4 + s * Q4 + q,
-                                 bh, amax_t);
-            po[0] = out;
+            single(q, s, bh);
         }
         if (MODE == 0 && em.aux != nullptr) {
             const unsigned int w = __reduce_max_sync(0xffffffffu, __float_as_uint(amax_t));
@@ -684,8 +698,27 @@ __device__ __forceinline__ bool run_strip(const RegParams& rp, const RegJob& job
         const int vnext = more && nrec > 0 ? fetch_var(job.var, i + 1, tid) : 0;
         if (nrec > 0) gather<MODE>(rp, job, sh, g_smem + cur * np, nrec, sh.v[cur].rec_t, tid);
         mail.asked = false;
-        // ---- inner quads: a thread slides both stencils across C positions of one quad
-        for (int it = tid; it < items; it += kT) {
+        // any quad: stencil centres clamped at the grid's edge (p) and at both edges of the strip (phi)
+        auto single = [&](int q, int s) {
+            const int cp = b.low ? max(s, 3) : min(s, ns - 4), cf = clampi(s, 3, ns - 4);
+            const float4* w = u.pc + cp * P4 + 1 + q;
+            const float4* f = u.ph + (cf - 3) * Q4 + q;
+            float4 X[7], F[7];
+#pragma unroll
+            for (int k = 0; k < 7; ++k) {
+                X[k] = w[k * P4];
+                F[k] = k == 3 ? make_float4(0.f, 0.f, 0.f, 0.f) : f[k * Q4];
+            }
+            const float4* zc = u.pc + (s + 3) * P4 + 1 + q;
+            strip_update<P>(kc, k1, u, q, s, X, F, zc[0], zc[-1], zc[1], u.ph[s * Q4 + q]);
+        };
+        // ---- inner quads: a thread slides both stencils across C positions of one quad, or takes single quads
+        for (int j = tid; C == 0 && j < items; j += kT) {
+            const int s = j / nqi;
+            if (j + kT >= items) mail.request(cur ^ 1, tid, i > 0);
+            single(b.qa + j - s * nqi, b.sa + s);
+        }
+        for (int it = tid; C > 0 && it < items; it += kT) {
             const int ch = it / nqi, q = b.qa + it - ch * nqi, s0 = b.sa + ch * C, n = min(C, b.sb - s0);
             const float4* w = u.pc + s0 * P4 + 1 + q;
             const float4* f = u.ph + (s0 - 3) * Q4 + q;
@@ -721,21 +754,11 @@ __device__ __forceinline__ bool run_strip(const RegParams& rp, const RegJob& job
         if (i > 0)
             ok = mail.receive(g_smem + cur * np, nullptr, cur ^ 1, rp.epoch + (unsigned int)i - 1u, rp.abort, tid);
         if (__syncthreads_or(!ok)) return false;
-        // ---- boundary quads: stencil centres clamped at the grid's edge (p) and at both edges of the strip (phi)
+        // ---- boundary quads
         for (int j = tid; j < nbound; j += kT) {
             int q = bq, s = bs;
             if (j != tid) boundary_quad(b, j, q, s);
-            const int cp = b.low ? max(s, 3) : min(s, ns - 4), cf = clampi(s, 3, ns - 4);
-            const float4* w = u.pc + cp * P4 + 1 + q;
-            const float4* f = u.ph + (cf - 3) * Q4 + q;
-            float4 X[7], F[7];
-#pragma unroll
-            for (int k = 0; k < 7; ++k) {
-                X[k] = w[k * P4];
-                F[k] = k == 3 ? make_float4(0.f, 0.f, 0.f, 0.f) : f[k * Q4];
-            }
-            const float4* zc = u.pc + (s + 3) * P4 + 1 + q;
-            strip_update<P>(kc, k1, u, q, s, X, F, zc[0], zc[-1], zc[1], u.ph[s * Q4 + q]);
+            single(q, s);
         }
         if (more && nrec > 0) store_var(&sh.v[cur ^ 1], vnext, tid);
         __syncthreads();
@@ -1057,7 +1080,7 @@ void item_shape(RegBlock* r, int nb) {
         r->sa = 3;
         r->sb = std::max(3, r->ns - 3);
     }
-    r->C = 1;
+    r->C = 0;
     if (r->type == kRegCorner) {
         r->items = (r->fb - r->fa) * (r->sb - r->sa);
         r->nbound = r->nf * r->ns - r->items;
@@ -1069,7 +1092,12 @@ void item_shape(RegBlock* r, int nb) {
     if (r->items > 0) {
         const int nch = std::max(1, std::min(nsi, kT / nqi));
         r->C = (nsi + nch - 1) / nch;
-        r->items = nqi * ((nsi + r->C - 1) / r->C);
+        // single quads where a column would be one or two long: a column's first quad costs 1050 cycles more than a
+        // single one's (200 x 249 window, 3000 steps: 19.8 -> 15.0 ms, 331 x 321 9.6 -> 7.0)
+        if (r->C <= 2)
+            r->C = 0;
+        else
+            r->items = nqi * ((nsi + r->C - 1) / r->C);
     }
 }
 
@@ -1083,7 +1111,11 @@ size_t region_floats(int P_, int type, int nf, int ns, int nslot, bool img) {
 }
 
 // Estimated cycles of a region's step: warp instructions over the four
-// schedulers, at least the chain of its longest thread.
+// schedulers, at least the chain of its longest thread, in both phases, and
+// its packets: the fixed round trip, a chain of one packet per kT, and a share
+// per packet.  That share (7 cycles) was taken where the windows that are all
+// latency stop gaining: 331 x 321 with C-PML on all sides 7.4, 7.0, 7.0 and
+// 6.4 ms with 1.7, 2.5, 4 and 7; 200 x 249 15.0, 15.0, 12.8 and 12.9.
 double region_cost(int type, int nf, int ns) {
     RegBlock r{};
     r.type = type;
@@ -1095,9 +1127,14 @@ double region_cost(int type, int nf, int ns) {
     auto phase = [](int items, double warp, double chain, double fixed) {
         return items > 0 ? std::max(std::ceil(items / 32.0) * warp, std::ceil(items / (double)kT) * chain) + fixed : 0.0;
     };
-    if (type == kRegCorner) return phase(r.items, 82, 950, 100) + phase(r.nbound, 100, 950, 400) + 700;
-    if (type == kRegStrip) return phase(r.items, r.C * 85.0, r.C * 650.0, 1000) + phase(r.nbound, 160, 1100, 400) + 900;
-    return phase(r.items, r.C * 62.0, r.C * 450.0, 400) + phase(r.nbound, 80, 800, 300) + 900;
+    const double pk = 2.0 * (nf + ns);  // packets each way
+    const double mail = 700 + 300 * std::ceil(pk / kT) + 7.0 * pk;
+    if (type == kRegCorner) return phase(r.items, 75, 860, 100) + phase(r.nbound, 60, 500, 500) + mail;
+    if (type == kRegStrip)
+        return (r.C > 0 ? phase(r.items, r.C * 85.0, r.C * 950.0, 550) : phase(r.items, 90, 900, 250)) +
+               phase(r.nbound, 80, 800, 350) + mail;
+    return (r.C > 0 ? phase(r.items, r.C * 52.0, r.C * 560.0, 1050) : phase(r.items, 70, 700, 250)) +
+           phase(r.nbound, 70, 700, 250) + mail;
 }
 
 struct Part {  // a rectangle of the padded grid cut into a x b regions

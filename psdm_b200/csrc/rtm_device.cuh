@@ -81,6 +81,9 @@ __device__ __forceinline__ float div_dt_common(const StepArgs& a, float x, bool&
 // its writes are visible.  (Triggering the dependent launch early made the
 // single-shot step slower: the waiting blocks take resident slots.)
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 __device__ __forceinline__ float comp(const float4& v, int r) {
     return r == 0 ? v.x : (r == 1 ? v.y : (r == 2 ? v.z : v.w));
@@ -112,21 +115,32 @@ __device__ __forceinline__ void quantize_part(const float* __restrict__ src, con
     if (blockIdx.x == 0 && tid == 0) *iscale = pow2f(-k);
     const float4* s4 = reinterpret_cast<const float4*>(src);
     uint2* d4 = reinterpret_cast<uint2*>(dst);
-    for (int i = blockIdx.x * NT + tid; i < n / 4; i += gridDim.x * NT) {
-        const float4 v = __ldg(s4 + i);
-        const float x0 = __fmul_rn(v.x, sc), x1 = __fmul_rn(v.y, sc), x2 = __fmul_rn(v.z, sc),
-                    x3 = __fmul_rn(v.w, sc);
-        uint2 o;
-        if (kind16 == 1) {
-            const __half2 a = __floats2half2_rn(x0, x1), b = __floats2half2_rn(x2, x3);
-            o.x = *reinterpret_cast<const unsigned int*>(&a);
-            o.y = *reinterpret_cast<const unsigned int*>(&b);
-        } else {
-            const __nv_bfloat162 a = __floats2bfloat162_rn(x0, x1), b = __floats2bfloat162_rn(x2, x3);
-            o.x = *reinterpret_cast<const unsigned int*>(&a);
-            o.y = *reinterpret_cast<const unsigned int*>(&b);
+    // kFly loads in flight a thread (3000 x 2619 window: 33.7 -> 33.2 us a
+    // step, one snapshot in four steps; 8 gain nothing more)
+    constexpr int kFly = 4;
+    const int st = gridDim.x * NT, m = n / 4;
+    for (int i0 = blockIdx.x * NT + tid; i0 < m; i0 += kFly * st) {
+        float4 v[kFly];
+#pragma unroll
+        for (int u = 0; u < kFly; ++u)
+            if (i0 + u * st < m) v[u] = __ldg(s4 + i0 + u * st);
+#pragma unroll
+        for (int u = 0; u < kFly; ++u) {
+            if (i0 + u * st >= m) break;
+            const float x0 = __fmul_rn(v[u].x, sc), x1 = __fmul_rn(v[u].y, sc), x2 = __fmul_rn(v[u].z, sc),
+                        x3 = __fmul_rn(v[u].w, sc);
+            uint2 o;
+            if (kind16 == 1) {
+                const __half2 a = __floats2half2_rn(x0, x1), b = __floats2half2_rn(x2, x3);
+                o.x = *reinterpret_cast<const unsigned int*>(&a);
+                o.y = *reinterpret_cast<const unsigned int*>(&b);
+            } else {
+                const __nv_bfloat162 a = __floats2bfloat162_rn(x0, x1), b = __floats2bfloat162_rn(x2, x3);
+                o.x = *reinterpret_cast<const unsigned int*>(&a);
+                o.y = *reinterpret_cast<const unsigned int*>(&b);
+            }
+            d4[i0 + u * st] = o;
         }
-        d4[i] = o;
     }
 }
 

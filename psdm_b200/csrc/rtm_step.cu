@@ -661,16 +661,43 @@ constexpr int smem_floats() {
     return tile_smem_cols(XS) * HZ;  // the p tile of an interior tile (boundary tiles use less)
 }
 
-template <int MODE>
+// One time step of one shot.
+//
+// MANY = false: about as many tiles as resident blocks (operands in L2).  The
+// step is latency: a block starts on the tile of its own number, so that the
+// counter is asked only for further ones (against asking it for the first
+// too: a shot of 3000 steps on a 200 x 249 window 54.0 -> 48.2 ms, of 2000 on
+// 1200 x 1136 40.8 -> 37.7).
+//
+// MANY = true: several tiles a block (launch_mode's rule), operands beyond L2.
+// The step is bound by loads in flight and by what the tiles leave idle, so
+//  * p1 and c2 come kRing columns ahead through the shared ring (RG);
+//  * every other step takes the interior tiles in reverse, so that a step
+//    begins with the columns the last one left in L2;
+//  * the C-PML and row-band tiles, a tenth of the cells but a quarter of the
+//    time when they end the step on their own (7.8 of 32 us), are spread
+//    evenly over the first half of the list;
+//  * the next step's blocks may be launched early (they wait for this grid).
+// 3000 x 2619 window, 16-bit snapshots of every fourth step, forward and
+// backward: 44.3 us a step before; ring and reversal 38.9, spread 34.4, early
+// launch 33.7, more loads in flight in the conversion 32.6 (FP32 snapshots of
+// every fourth step: 39.2 -> 27.8).  The p, p1 and c2 of a step alone take
+// 21 us from HBM.  What did not help: wider tiles (48 columns 31.7 against
+// 31.2 of 32), 6 or 4 blocks a multiprocessor, a ring of 4 or 6 columns, the
+// next tile's number asked for ahead (the last tiles end later: 27.9 -> 30.2),
+// streaming hints on the snapshots and the image.
+template <int MODE, bool MANY>
 __global__ void __launch_bounds__(NT, 5) step_kernel(const StepArgs a) {
     extern __shared__ __align__(128) float sm[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ int tile_id;
     const int tid = threadIdx.y * 32 + threadIdx.x;
     grid_dependency_wait();
+    if (MANY) grid_launch_dependents();
     if (tid == 0) {
         mbar_init(&bar, 1);
         s_blk_amax = 0u;
+        if (!MANY) tile_id = blockIdx.x;
     }
     // Receivers of the previous step (p is that step's p3, read-only during
     // this step): spread over the blocks, a receiver per thread, loaded before
@@ -691,28 +718,41 @@ __global__ void __launch_bounds__(NT, 5) step_kernel(const StepArgs a) {
         }
     }
     if (MODE == 0 && a.q_src != nullptr) quantize_part(a.q_src, a.q_amax, a.q_dst, a.q_iscale, a.q_n, a.kind16, tid);
-    // Persistent blocks take tiles in order (heaviest rect types first) from
-    // this step's counter; the other counter is cleared for the next step.
+    // Persistent blocks take tiles from this step's counter, in order (heaviest
+    // rect types first) or spread; the other counter is cleared for the next step.
     if (blockIdx.x == 0 && tid == 0) a.tile_counter[a.counter_sel ^ 1] = 0;
     __syncthreads();
     uint32_t phase = 0;
-    const int total = a.r_first[a.nrect];
+    const int total = a.r_first[a.nrect], grid = gridDim.x;
+    int nin = 0;  // interior tiles, the first of the list
+    if (MANY) {
+        int r = 0;
+        while (r < a.nrect && a.r_type[r] == 0) ++r;
+        nin = a.r_first[r];
+    }
+    const int nbd = total - nin, span = max(total / 2, nbd);  // nbd others among the first span tiles
     for (;;) {
-        if (tid == 0) tile_id = atomicAdd(a.tile_counter + a.counter_sel, 1);
+        if (MANY && tid == 0) tile_id = atomicAdd(a.tile_counter + a.counter_sel, 1);
         __syncthreads();
-        const int b = tile_id;
+        int b = tile_id;
         if (b >= total) {
             if (MODE == 0 && tid == 0 && a.field_amax != nullptr && s_blk_amax != 0u)
                 atomicMax(a.field_amax, s_blk_amax);
             if (MODE == 0 && rec_i >= 0) a.rec_out[(size_t)rec_i * a.rec_ld + a.rec_t] = rec_v;
             return;
         }
+        if (MANY) {
+            const int k0 = min(nbd, (int)((long long)b * nbd / span)),
+                      k1 = min(nbd, (int)((long long)(b + 1) * nbd / span));
+            b = k1 > k0 ? nin + k0 : b - k0;
+        }
         int r = 0;
         while (r + 1 < a.nrect && b >= a.r_first[r + 1]) ++r;
-        const int t = b - a.r_first[r];
+        int t = b - a.r_first[r];
+        if (MANY && a.counter_sel && a.r_type[r] == 0) t = a.r_first[r + 1] - a.r_first[r] - 1 - t;
         switch (a.r_type[r]) {
             case 0:
-                if (!interior_tile<MODE, xs_one<MODE>()>(a, sm, &bar, phase, r, t)) return;
+                if (!interior_tile<MODE, xs_one<MODE>(), false, MANY>(a, sm, &bar, phase, r, t)) return;
                 break;
             case 1:
                 if (!xband_tile<MODE, xxs<MODE, false>()>(a, sm, r, t)) return;
@@ -725,6 +765,8 @@ __global__ void __launch_bounds__(NT, 5) step_kernel(const StepArgs a) {
             default: generic_tile<MODE>(a, sm, r, t); break;
         }
         __syncthreads();  // shared tile and tile_id are reused
+        if (!MANY && tid == 0)
+            tile_id = grid >= total ? total : grid + atomicAdd(a.tile_counter + a.counter_sel, 1);
     }
 }
 
@@ -1040,17 +1082,20 @@ void plan_tiles(StepArgs* a, const int* row_slot_host, bool batched, bool forwar
 }
 
 // Dynamic shared memory of the one-shot step kernel: an interior tile's p
-// tile, or a staged z-strip tile.
-constexpr int step_smem_floats() { return smem_floats<XS_ONE>() > kZsFloats ? smem_floats<XS_ONE>() : kZsFloats; }
+// tile (and ring), or a staged z-strip tile.
+constexpr int step_smem_floats(bool many) {
+    const int in = smem_floats<XS_ONE>() + (many ? 4 * 2 * kRing * NT : 0);
+    return in > kZsFloats ? in : kZsFloats;
+}
 
-template <int MODE>
+template <int MODE, bool MANY>
 int blocks_per_sm() {
     static int nb = 0;
     if (nb == 0) {
-        const int bytes = step_smem_floats() * (int)sizeof(float);
-        cudaFuncSetAttribute(step_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        const int bytes = step_smem_floats(MANY) * (int)sizeof(float);
+        cudaFuncSetAttribute(step_kernel<MODE, MANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         int n = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, step_kernel<MODE>, NT, bytes);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, step_kernel<MODE, MANY>, NT, bytes);
         nb = n > 0 ? n : 1;
     }
     return nb;
@@ -1069,11 +1114,10 @@ int batch_blocks_per_sm() {
     return nb;
 }
 
-template <int MODE>
-int launch_mode(const StepArgs& a, cudaStream_t stream) {
-    if (a.ixb != NWARP * xxs<MODE, false>()) return (int)cudaErrorInvalidValue;  // a plan for another launch form
-    const int bytes = step_smem_floats() * (int)sizeof(float);
-    const dim3 grid(min(a.r_first[a.nrect], a.num_sms * blocks_per_sm<MODE>()));
+template <int MODE, bool MANY>
+int launch_mode_t(const StepArgs& a, cudaStream_t stream) {
+    const int bytes = step_smem_floats(MANY) * (int)sizeof(float);
+    const dim3 grid(min(a.r_first[a.nrect], a.num_sms * blocks_per_sm<MODE, MANY>()));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(32, NWARP);
@@ -1084,7 +1128,19 @@ int launch_mode(const StepArgs& a, cudaStream_t stream) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return (int)cudaLaunchKernelEx(&cfg, step_kernel<MODE>, a);
+    return (int)cudaLaunchKernelEx(&cfg, step_kernel<MODE, MANY>, a);
+}
+
+// MANY where a step has more tiles than resident blocks.  Measured, a step of
+// forward and backward with 16-bit / FP32 snapshots, MANY against not: 1200 x
+// 1119 (0.8-1.0 waves) 11.1 / 10.5 against 10.2 / 9.0 us; 1200 x 1419 (1.0-1.2)
+// 11.9 / 11.1 against 12.6 / 11.6; 2100 x 2219 20.1 / 17.6 against 25.6 / 20.1;
+// 3000 x 2619 32.6 / 27.8 against 45.8 / 39.5.
+template <int MODE>
+int launch_mode(const StepArgs& a, cudaStream_t stream) {
+    if (a.ixb != NWARP * xxs<MODE, false>()) return (int)cudaErrorInvalidValue;  // a plan for another launch form
+    const bool many = a.r_first[a.nrect] > a.num_sms * blocks_per_sm<MODE, false>();
+    return many ? launch_mode_t<MODE, true>(a, stream) : launch_mode_t<MODE, false>(a, stream);
 }
 
 template <int MODE>
@@ -1118,7 +1174,8 @@ int launch_pass_t(const PassParams& pp, int grid, cudaStream_t stream) {
 int prepare_step_kernels() {
     // Kernel attributes and occupancy are set up once, outside any stream
     // capture.
-    return (blocks_per_sm<0>() > 0 && blocks_per_sm<1>() > 0 && blocks_per_sm<2>() > 0 &&
+    return (blocks_per_sm<0, false>() > 0 && blocks_per_sm<1, false>() > 0 && blocks_per_sm<2, false>() > 0 &&
+            blocks_per_sm<0, true>() > 0 && blocks_per_sm<1, true>() > 0 && blocks_per_sm<2, true>() > 0 &&
             batch_blocks_per_sm<-1>() > 0 && batch_blocks_per_sm<0>() > 0 && batch_blocks_per_sm<1>() > 0 &&
             batch_blocks_per_sm<2>() > 0 && pass_blocks_per_sm_t<0>() >= 0 && pass_blocks_per_sm_t<1>() >= 0 &&
             pass_blocks_per_sm_t<2>() >= 0)

@@ -857,12 +857,16 @@ __global__ void __launch_bounds__(NT, 5) batch_step_kernel(const BatchParams bp)
     for (;;) {
         if (tid == 0) tile_id = atomicAdd(bp.counter + bp.counter_sel, 1);
         __syncthreads();
-        const int b = tile_id;
+        int b = tile_id;
         if (b >= total) {
             if (tid == 0 && cur >= 0 && bp.mode[cur] == 0 && sa.field_amax != nullptr && s_blk_amax != 0u)
                 atomicMax(sa.field_amax, s_blk_amax);
             return;
         }
+        // every other launch takes the list backwards: it begins with what the last one left in L2, and
+        // boundary tiles overlap interior ones (FP16 shots of 3000 x 2620: 3 in flight 1.09 -> 1.15 shots/s,
+        // 8 with checkpoints 0.859 -> 0.879)
+        if (bp.counter_sel) b = total - 1 - b;
         int s = 0;
         while (s + 1 < bp.nslots && b >= bp.first[s + 1]) ++s;
         if (s != cur) {  // every thread takes the same branch

@@ -90,16 +90,16 @@ def algorithmic_bytes_mixed(ny, nx_w, dpml, fs, ks):
     return base + 10 * g["n_int"] / ks, base + 18 * g["n_int"] / ks, g
 
 
-def profiled_traffic(which: str):
-    """DRAM bytes (read + write) per launch of the step kernel from the ncu
-    capture summarised in profiles/ (a `traffic_bytes_per_launch:` line), or
-    None if there is none."""
+def profiled_traffic(which: str, name="step_kernel_config2_ncu_full.md", key="traffic_bytes_per_launch"):
+    """DRAM bytes (read + write) from an ncu capture summarised in profiles/
+    (its `key:` line), or None if there is none: by default those of a launch
+    of the step kernel."""
     import re
-    p = os.path.join(ROOT, "profiles", "step_kernel_config2_ncu_full.md")
+    p = os.path.join(ROOT, "profiles", name)
     if not os.path.exists(p):
         return None
     with open(p) as f:
-        m = re.search(r"traffic_bytes_per_launch:\s*fwd=(\d+)\s+bwd=(\d+)", f.read())
+        m = re.search(key + r":\s*fwd=(\d+)\s+bwd=(\d+)", f.read())
     if not m:
         return None
     return int(m.group(1) if which == "fwd" else m.group(2))
@@ -244,10 +244,13 @@ def run_reference(args):
 # slots = 0 is one shot at a time through psdm_rtm_shot_device, otherwise
 # psdm_rtm_batch_device with that many shots in flight; precision 1 / 2 =
 # binary16 / bfloat16 snapshots every ks steps; ckpt = checkpoint interval of
-# FP32 shots; spl = time steps per kernel launch.
+# FP32 shots; spl = time steps per kernel launch; pass_form = launch form set
+# explicitly.
 FORMS = [
     dict(name="fp32_two_steps", precision=0, ks=1, slots=0, spl=2),
-    dict(name="fp32_resident", precision=0, ks=1, slots=0, pass_form=2),
+    dict(name="fp32_steps", precision=0, ks=1, slots=0, pass_form=0, launch="one launch per time step"),
+    dict(name="fp32_resident", precision=0, ks=1, slots=0, pass_form=2,
+         launch="one cooperative launch per pass, regions resident in shared memory, step counters"),
     dict(name="fp16_ks4", precision=1, ks=4, slots=0),
     dict(name="batch_fp16_ks4", precision=1, ks=4, slots=8),
     dict(name="batch_bf16_ks4", precision=2, ks=4, slots=8),
@@ -329,7 +332,19 @@ def synth_model_cached():
     return _VEL
 
 
-def time_forms(engine, torch, dev, stream, d_src, items, names, ref_value):
+def _form_engine(engine, stream, dev, pass_form):
+    """The engine a form runs on: an engine of its own for an explicit launch form, which an engine keeps
+    once it is set."""
+    from psdm_b200 import rtm
+    if pass_form is None:
+        return engine
+    e = rtm.Engine(dev.index)
+    e.set_stream(stream.cuda_stream)
+    e.set_pass_launch(pass_form)
+    return e
+
+
+def time_forms(plain, torch, dev, stream, d_src, items, names, ref_value):
     """Shots/s of each named form on the workload's shots (inputs in HBM)."""
     from psdm_b200 import rtm
     out = {}
@@ -341,10 +356,10 @@ def time_forms(engine, torch, dev, stream, d_src, items, names, ref_value):
         prm = rtm.Params(dPML=DPML, fs=1, strategy=1, precision=precision)
         ckpt = f.get("ckpt", 0)
         n = 2 * slots if slots else 4
+        engine = _form_engine(plain, stream, dev, f.get("pass_form"))
         engine.set_checkpointing(ckpt)
         engine.set_reconstruction(f.get("recon", False))
         engine.set_steps_per_launch(f.get("spl", 1))
-        engine.set_pass_launch(f.get("pass_form", 0))
         sel = [(items[i % len(items)], outs[i % len(outs)]) for i in range(n)]
 
         def run(k):
@@ -370,7 +385,6 @@ def time_forms(engine, torch, dev, stream, d_src, items, names, ref_value):
         engine.set_checkpointing(0)
         engine.set_reconstruction(False)
         engine.set_steps_per_launch(1)
-        engine.set_pass_launch(0)
         v = n / (e0.elapsed_time(e1) / 1e3)
         out[name] = {"shots_per_s": v, "vs_plain": v / ref_value, "shots": n,
                      "slots": engine.batch_slots() if slots else 1, "precision": ["f32", "fp16", "bf16"][precision],
@@ -381,8 +395,9 @@ def time_forms(engine, torch, dev, stream, d_src, items, names, ref_value):
             out[name]["steps_per_launch"] = f["spl"]
         if f.get("recon"):
             out[name]["source_wavefield"] = "reconstructed from a saved 3-cell band"
-        if f.get("pass_form"):
-            out[name]["launch"] = "one cooperative launch per pass, regions resident in shared memory"
+        if "pass_form" in f:
+            out[name]["launch"] = f["launch"]
+            engine.close()
     return out
 
 
@@ -436,11 +451,11 @@ def time_config1(engine, torch, dev, stream, peak, with_cpu, mixed=False):
                           d_vp=torch.from_numpy(vmw).to(dev), d_obs=torch.from_numpy(obs).to(dev),
                           d_img=torch.zeros((nx_w, ny), dtype=torch.float32, device=dev)))
 
-    def one_at_a_time(prm=prm, ks=1):
+    def one_at_a_time(prm=prm, ks=1, e=engine):
         for it in items:
-            engine.rtm_shot_device(prm, it["nxSou"], it["nySou"], it["nxRec"], it["nyRec"], d_src.data_ptr(),
-                                   it["d_obs"].data_ptr(), dd, dt, ny, nx, it["nx_w"], it["d_vp"].data_ptr(),
-                                   ADDED_SPACE, ks, nt, nt, nt, 0, 1, 0, it["d_img"].data_ptr())
+            e.rtm_shot_device(prm, it["nxSou"], it["nySou"], it["nxRec"], it["nyRec"], d_src.data_ptr(),
+                              it["d_obs"].data_ptr(), dd, dt, ny, nx, it["nx_w"], it["d_vp"].data_ptr(),
+                              ADDED_SPACE, ks, nt, nt, nt, 0, 1, 0, it["d_img"].data_ptr())
 
     def batched(prm=prm, ks=1):
         descs = [dict(nxSou=it["nxSou"], nySou=it["nySou"], nxRec=it["nxRec"], nyRec=it["nyRec"], nx_w=it["nx_w"],
@@ -456,13 +471,14 @@ def time_config1(engine, torch, dev, stream, peak, with_cpu, mixed=False):
                                             len(items), cells, (fb + bb) * (nt - 1), peak)
     out["gpu_batched_4"] = _config_line("config1", _shot_rate(torch, dev, stream, batched, len(items)), len(items),
                                         cells, (fb + bb) * (nt - 1), peak)
-    engine.set_pass_launch(2)  # each pass one launch, regions resident in shared memory
+    resident = _form_engine(engine, stream, dev, 2)
     try:
         out["gpu_resident_one_at_a_time"] = _config_line(
-            "config1", _shot_rate(torch, dev, stream, one_at_a_time, len(items)), len(items), cells,
-            (fb + bb) * (nt - 1), peak, launch="one cooperative launch per pass, regions resident in shared memory")
+            "config1", _shot_rate(torch, dev, stream, lambda: one_at_a_time(e=resident), len(items)), len(items), cells,
+            (fb + bb) * (nt - 1), peak,
+            launch="one cooperative launch per pass, regions resident in shared memory, step counters")
     finally:
-        engine.set_pass_launch(0)
+        resident.close()
     if with_cpu:
         ctx = mp.get_context("spawn")
         t0 = time.perf_counter()
@@ -721,17 +737,18 @@ def run_gpu(args):
     ms_max = float(ms_t.item())
     value = world * args.steps / (ms_max / 1e3)
 
-    # roofline of the dominant kernel (per-launch time from CUDA events)
+    # roofline of the dominant pass (time per step from CUDA events)
     nx_w0 = items[args.warmup]["nx_w"]
     fwd_b, bwd_b, g = algorithmic_bytes(NY, nx_w0, DPML, 1)
     fwd_us = st["fwd_ms"] * 1e3 / max(st["fwd_steps"], 1)
     bwd_us = st["bwd_ms"] * 1e3 / max(st["bwd_steps"], 1)
     dom = "bwd" if st["bwd_ms"] >= st["fwd_ms"] else "fwd"
     peak, peak_kind = _peaks()
-    bytes_dom = bwd_b if dom == "bwd" else fwd_b
+    # the region form keeps the wavefield, c2 and the image on the chip: a step moves its snapshot
     us_dom = bwd_us if dom == "bwd" else fwd_us
-    achieved = bytes_dom / (us_dom * 1e-6) / 1e9
-    traffic = profiled_traffic(dom)
+    achieved = 4 * g["n_int"] / (us_dom * 1e-6) / 1e9
+    one_step = (bwd_b if dom == "bwd" else fwd_b) / (us_dom * 1e-6) / 1e9
+    traffic = profiled_traffic(dom, "region_kernel_config2_ncu.md", "traffic_bytes_per_step")
 
     # end-to-end through the C ABI with pinned host buffers
     e2e = None
@@ -805,8 +822,8 @@ def run_gpu(args):
                 "gcell_upd_per_s": gcell,
                 "kernel": {"fwd_us_per_step": fwd_us, "bwd_us_per_step": bwd_us, "fwd_bytes": fwd_b,
                            "bwd_bytes": bwd_b},
-                "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                             "frac": achieved / peak, "traffic": traffic, "kernel": f"step_kernel<{dom}>",
+                "roofline": {"bound": "shared memory and issue", "achieved": achieved, "peak": peak, "unit": "GB/s",
+                             "frac": achieved / peak, "one_step_form_gbs": one_step, "traffic": traffic, "kernel": f"region_kernel<{dom}>, per time step",
                              "peak_kind": peak_kind},
                 "gpu_launches": int(st["launches"]),
                 "clocks": clk.summary(),

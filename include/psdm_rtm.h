@@ -220,9 +220,10 @@ int psdm_engine_set_checkpointing(psdm_engine* e, int32_t interval);
 int psdm_engine_set_reconstruction(psdm_engine* e, int32_t on);
 /*
  * Launch form of one shot's passes (psdm_rtm_shot, psdm_model_shot and their
- * device variants).  Until it is set, a forward or plain backward pass runs
- * as one cooperative launch of one block per region of the grid where the
- * grid fits the device's shared memory (the interior, C-PML strips and
+ * device variants).  Until it is set, every pass (plain, mixed-precision,
+ * checkpointed, and those of the batched calls, several shots side by side)
+ * runs as one cooperative launch of one block per region of the grid where
+ * the grid fits the device's shared memory (the interior, C-PML strips and
  * corners cut separately, edges exchanged as tagged packets), and others as 0
  * does.  1 runs a pass whose steps allow it as one cooperative
  * launch in which each tile advances as soon as its neighbours finished the
@@ -232,7 +233,8 @@ int psdm_engine_set_reconstruction(psdm_engine* e, int32_t on);
  * only the ring with its neighbours (grids that fit the device's blocks;
  * others fall back to one launch per step); 0 launches one kernel
  * per time step (replayed from a CUDA graph).  Same results bit for bit.
- * Passes with the mixed-precision snapshots always use one launch per step.
+ * With a form set, passes with the mixed-precision snapshots use one launch
+ * per step.
  * Values other than 0, 1 and 2 return PSDM_ERR_ARG.
  */
 int psdm_engine_set_pass_launch(psdm_engine* e, int32_t on);
@@ -243,8 +245,8 @@ int psdm_engine_set_pass_launch(psdm_engine* e, int32_t on);
  * step; 2 advances each tile two steps per launch, level n+1 computed on the
  * tile and a 3-cell ring in shared memory, so that the wavefield crosses HBM
  * and the launch queue half as often.  Same results bit for bit.  On the
- * B200 the one-step form is currently the faster (see psdm_engine_autotune,
- * which times both).  The cooperative pass launch
+ * B200 the passes that 1 allows are currently the faster (see
+ * psdm_engine_autotune, which times both).  The cooperative pass launch
  * (psdm_engine_set_pass_launch) and checkpointed shots use one step per
  * launch; reconstruction (psdm_engine_set_reconstruction) uses two.
  */

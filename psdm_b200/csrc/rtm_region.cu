@@ -30,7 +30,7 @@
 //
 // Measured on the B200 (a shot, against one launch per step): 1200 x 1136
 // window, 8000 steps 89.0 ms against 164.5 (forward step 10.4 -> 5.0 us,
-// backward 9.4 -> 6.2); 200 x 249, 3000 steps 13.0 against 53.4; 331 x 321
+// backward 9.4 -> 6.1); 200 x 249, 3000 steps 13.0 against 53.4; 331 x 321
 // with C-PML on all sides, 1501 steps 6.4 against 39.9; 36 x 64, 260 steps
 // 1.22 against 4.51.  12 warps of up to 168 registers: 16 warps spill the
 // column loops (model of the first window 24.3 against 19.5 ms), and two

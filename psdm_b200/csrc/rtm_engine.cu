@@ -1608,10 +1608,15 @@ void mixed_backward_args(const MixedBufs& mb, int nt, const float* h_w, std::vec
 int mixed_stage(psdm_engine* e, size_t fstride, int nsnap, size_t bytes, const std::string& tag, float** stage,
                 int* nstage) {
     *nstage = 0;
-    size_t fr = 0, tot = 0;
-    CUDA_TRY(cudaMemGetInfo(&fr, &tot));
     const size_t have = e->bufs[("reg_staging" + tag)].bytes;
-    const size_t room = std::max(have, std::min(bytes, fr / 8));
+    size_t room = have;
+    // the driver is asked only where the buffer is to grow: the query took tens of milliseconds at times
+    // (8 FP16 shots of 1200 x 1136, 1200 steps: passes of 140-200 ms among those of 102)
+    if (have < std::min(bytes, fstride * sizeof(float) * (size_t)std::max(nsnap, 1))) {
+        size_t fr = 0, tot = 0;
+        CUDA_TRY(cudaMemGetInfo(&fr, &tot));
+        room = std::max(have, std::min(bytes, fr / 8));
+    }
     const int n = (int)std::min<size_t>(room / (fstride * sizeof(float)), (size_t)std::max(nsnap, 1));
     if (n < std::min(4, std::max(nsnap, 1))) return PSDM_OK;
     TRY(e->get(("reg_staging" + tag).c_str(), fstride * (size_t)n, stage));

@@ -105,10 +105,10 @@ struct psdm_engine {
     // as one region launch each where the grid fits (rtm_region.cu).
     bool use_regions = true;
     // Region plans by (ny, nx, dPML, fs, regions, pitch), each with its lists in
-    // buffers of its own; the oldest gives way.
+    // buffers of its own.  A group of shots holds a plan a shot while it is
+    // prepared, up to kMaxSlots of them.
     struct RegSlot {
-        std::array<int, 6> key{};
-        bool used = false, fits = false;
+        bool fits = false;
         RegPlan plan;
         RegBlock* d_blocks = nullptr;
         RegPair* d_pub = nullptr;
@@ -116,7 +116,7 @@ struct psdm_engine {
     };
     static constexpr int kRegPlans = 2 * kMaxSlots;
     RegSlot reg_plans[kRegPlans];
-    int reg_next = 0;
+    KeyedSlots<std::array<int, 6>, kRegPlans> reg_keys;
     std::map<std::array<int, 5>, double> reg_cost;  // region_step_cost by (ny, nx, dPML, fs, regions)
     std::map<std::string, cudaEvent_t> reg_staged;  // copies out of a staging buffer done
     unsigned int reg_epoch = 1;  // tag of the next region launch's first step
@@ -188,6 +188,7 @@ struct psdm_engine {
         for (auto& k : pass_key) k.clear();
         for (auto& k : res_key) k.clear();
         for (RegSlot& r : reg_plans) r = RegSlot{};
+        reg_keys = {};
         reg_board = nullptr;
         for (auto& kv : fft_plans) destroy_fft_plans(kv.second.data());
         fft_plans.clear();
@@ -752,36 +753,38 @@ CoopOrder& coop_order() {
 }
 
 // The plan of a grid for `regions` blocks, made and uploaded on first use.
-// *out = null if the grid does not fit.
+// *out = null if the grid does not fit.  The pointer holds for the next
+// kRegPlans - 1 plans asked for.
 int region_plan(psdm_engine* e, const Grid& g, int fs, int regions, int pitch, psdm_engine::RegSlot** out) {
-    const std::array<int, 6> key = {g.ny, g.nx, g.dPML, fs, regions, pitch};
     *out = nullptr;
-    for (auto& r : e->reg_plans)
-        if (r.used && r.key == key) {
-            if (r.fits) *out = &r;
-            return PSDM_OK;
-        }
-    const int k = e->reg_next;
+    bool held = false;
+    const int k = e->reg_keys.take({g.ny, g.nx, g.dPML, fs, regions, pitch}, &held);
     auto& r = e->reg_plans[k];
-    e->reg_next = (k + 1) % psdm_engine::kRegPlans;
-    r = psdm_engine::RegSlot{};
-    r.key = key;
-    r.fits = plan_regions(g, fs, regions, region_max_floats(), &r.plan, pitch);
-    if (!r.fits) {
-        r.used = true;
+    if (held) {
+        if (r.fits) *out = &r;
         return PSDM_OK;
     }
-    const std::string t = std::to_string(k);
-    TRY(e->get(("reg_blocks" + t).c_str(), r.plan.blocks.size(), &r.d_blocks));
-    TRY(e->get(("reg_pub" + t).c_str(), std::max<size_t>(r.plan.pub.size(), 1), &r.d_pub));
-    TRY(e->get(("reg_rcv" + t).c_str(), std::max<size_t>(r.plan.rcv.size(), 1), &r.d_rcv));
-    CUDA_TRY(cudaMemcpyAsync(r.d_blocks, r.plan.blocks.data(), r.plan.blocks.size() * sizeof(RegBlock),
-                             cudaMemcpyHostToDevice, e->stream));
-    CUDA_TRY(cudaMemcpyAsync(r.d_pub, r.plan.pub.data(), r.plan.pub.size() * sizeof(RegPair), cudaMemcpyHostToDevice,
-                             e->stream));
-    CUDA_TRY(cudaMemcpyAsync(r.d_rcv, r.plan.rcv.data(), r.plan.rcv.size() * sizeof(int), cudaMemcpyHostToDevice,
-                             e->stream));
-    r.used = true;  // once the uploads are queued
+    r = psdm_engine::RegSlot{};
+    if (!plan_regions(g, fs, regions, region_max_floats(), &r.plan, pitch)) return PSDM_OK;
+    auto upload = [&]() -> int {
+        const std::string t = std::to_string(k);
+        TRY(e->get(("reg_blocks" + t).c_str(), r.plan.blocks.size(), &r.d_blocks));
+        TRY(e->get(("reg_pub" + t).c_str(), std::max<size_t>(r.plan.pub.size(), 1), &r.d_pub));
+        TRY(e->get(("reg_rcv" + t).c_str(), std::max<size_t>(r.plan.rcv.size(), 1), &r.d_rcv));
+        CUDA_TRY(cudaMemcpyAsync(r.d_blocks, r.plan.blocks.data(), r.plan.blocks.size() * sizeof(RegBlock),
+                                 cudaMemcpyHostToDevice, e->stream));
+        CUDA_TRY(cudaMemcpyAsync(r.d_pub, r.plan.pub.data(), r.plan.pub.size() * sizeof(RegPair),
+                                 cudaMemcpyHostToDevice, e->stream));
+        CUDA_TRY(cudaMemcpyAsync(r.d_rcv, r.plan.rcv.data(), r.plan.rcv.size() * sizeof(int), cudaMemcpyHostToDevice,
+                                 e->stream));
+        return PSDM_OK;
+    };
+    const int rc = upload();
+    if (rc != PSDM_OK) {
+        e->reg_keys.drop(k);
+        return rc;
+    }
+    r.fits = true;
     *out = &r;
     return PSDM_OK;
 }
@@ -2577,6 +2580,8 @@ int batch_group(psdm_engine* e, const BatchJob& j, int first, int most) {
 // is launched, if one of them does not fit.
 int batch_group_run(psdm_engine* e, const BatchJob& j, std::vector<BatchSlot>& slots, int first, int n) {
     const bool mixed = j.prm->precision != PSDM_PREC_FP32;
+    // plans of the group's first shots outlast the making of the others'
+    static_assert(psdm_engine::kRegPlans >= kMaxSlots, "a group holds a plan a shot");
     const std::vector<int> share = batch_shares(e, j, first, n);
     std::vector<RegSpec> fw(n), bw(n);
     std::vector<float*> stage(n, nullptr);

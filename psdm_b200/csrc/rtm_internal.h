@@ -509,6 +509,32 @@ struct RegLists {
     std::vector<RegPair> inj, rec;
     size_t floats = 0, floats_img = 0;  // shared floats with the source buffers, and with the image
 };
+// Which of N slots holds a key.  The slot taken longest ago gives way, so the
+// slots of the last N keys taken stay theirs: a caller that holds several
+// slots at once (the shots of a group) takes no more than N.
+template <class Key, int N>
+struct KeyedSlots {
+    Key key[N] = {};
+    unsigned long long taken[N] = {};  // when last taken, 0: empty
+    unsigned long long now = 0;
+    // The slot of `k`; *held tells whether it held it already.
+    int take(const Key& k, bool* held) {
+        int at = 0;
+        for (int i = 0; i < N; ++i) {
+            if (taken[i] != 0 && key[i] == k) {
+                taken[i] = ++now;
+                *held = true;
+                return i;
+            }
+            if (taken[i] < taken[at]) at = i;
+        }
+        key[at] = k;
+        taken[at] = ++now;
+        *held = false;
+        return at;
+    }
+    void drop(int i) { taken[i] = 0; }
+};
 // Regions and packets of a padded grid for at most max_regions blocks of
 // max_floats shared floats, with columns of `pitch` (0: the cheaper one).
 // False if the grid does not fit.

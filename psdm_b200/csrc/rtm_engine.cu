@@ -2425,7 +2425,20 @@ int batch_program_ckpt(psdm_engine* e, const BatchJob& j, BatchSlot& sl, int i, 
     return PSDM_OK;
 }
 
-// Shot `i`'s inputs, state and window in slot `sl`.
+// Host variant: copy a finished image out of the slot's page-locked buffer.
+int batch_flush(psdm_engine* e, BatchSlot& sl) {
+    if (!sl.h_out) return PSDM_OK;
+    CUDA_TRY(cudaEventSynchronize(sl.staged));
+    void* h_img = nullptr;
+    const size_t bytes = (size_t)sl.out_ny * sl.out_nx * sizeof(float);
+    TRY(e->get_pinned(("himg" + sl.tag).c_str(), bytes, &h_img));
+    std::memcpy(sl.h_out, h_img, bytes);
+    sl.h_out = nullptr;
+    return PSDM_OK;
+}
+
+// Shot `i`'s inputs, state and window in slot `sl`, whose last shot's image
+// leaves first, whichever route that shot took.
 int batch_inputs(psdm_engine* e, const BatchJob& j, BatchSlot& sl, int i, const float** p_vp, const float** p_tgt,
                  WinGeom* w) {
     const psdm_shot& sh = j.shots[i];
@@ -2436,6 +2449,7 @@ int batch_inputs(psdm_engine* e, const BatchJob& j, BatchSlot& sl, int i, const 
     d_vp = sh.Vp_w;
     d_tgt = sh.Data_target;
     const size_t nvp = (size_t)ny * nx_w, ntgt = (size_t)sh.NumRec * sh.nt_taper;
+    TRY(batch_flush(e, sl));
     // The slot's page-locked staging is reused only once its previous
     // copies have completed.
     CUDA_TRY(cudaEventSynchronize(sl.staged));
@@ -2462,7 +2476,6 @@ int batch_inputs(psdm_engine* e, const BatchJob& j, BatchSlot& sl, int i, const 
     sl.out_ny = ny;
     sl.out_nx = nx_w;
     sl.d_out = j.host_io ? nullptr : sh.PSDM_w;
-    sl.h_out = nullptr;
     return PSDM_OK;
 }
 
@@ -2478,18 +2491,6 @@ int batch_start(psdm_engine* e, const BatchJob& j, BatchSlot& sl, int i) {
     CUDA_TRY(cudaEventRecord(sl.staged, e->stream));
     CUDA_TRY(cudaMemsetAsync(sl.d_imgp, 0, sl.s.g.field_cells() * sizeof(float), e->stream));
     sl.shot = i;
-    return PSDM_OK;
-}
-
-// Host variant: copy a finished image out of the slot's page-locked buffer.
-int batch_flush(psdm_engine* e, BatchSlot& sl) {
-    if (!sl.h_out) return PSDM_OK;
-    CUDA_TRY(cudaEventSynchronize(sl.staged));
-    void* h_img = nullptr;
-    const size_t bytes = (size_t)sl.out_ny * sl.out_nx * sizeof(float);
-    TRY(e->get_pinned(("himg" + sl.tag).c_str(), bytes, &h_img));
-    std::memcpy(sl.h_out, h_img, bytes);
-    sl.h_out = nullptr;
     return PSDM_OK;
 }
 
@@ -2590,7 +2591,6 @@ int batch_group_run(psdm_engine* e, const BatchJob& j, std::vector<BatchSlot>& s
     for (int k = 0; k < n; ++k) {
         BatchSlot& sl = slots[k];
         const psdm_shot& sh = j.shots[first + k];
-        TRY(batch_flush(e, sl));
         const float *d_vp = nullptr, *d_tgt = nullptr;
         WinGeom w;
         TRY(batch_inputs(e, j, sl, first + k, &d_vp, &d_tgt, &w));
@@ -2740,10 +2740,7 @@ int run_batch(psdm_engine* e, const BatchJob& j, int max_slots) {
                 e->bwd_steps += sl.bwd_steps;
                 TRY(batch_finish(e, j, sl));
                 sl.shot = -1;
-                if (next < j.nshots) {
-                    TRY(batch_flush(e, sl));
-                    TRY(batch_start(e, j, sl, next++));
-                }
+                if (next < j.nshots) TRY(batch_start(e, j, sl, next++));
                 continue;
             }
             const SlotOp& op = sl.ops[sl.pc];

@@ -313,6 +313,13 @@ int psdm_engine_check_wait_timeout(psdm_engine* e);
  * multiple of 4; q holds 2 n floats.
  */
 int psdm_engine_dt_quotients(psdm_engine* e, float dt, const float* x, int32_t n, float* q);
+/*
+ * The same of the region launches: q = (p3 - p1) * 0.5 / dt in FP32 for n
+ * host cells of levels p3 and p1, every operation rounded to nearest, as a
+ * snapshot is stored (src/solver_ac_forward_ram.f90:485).  n is a positive
+ * multiple of 4.
+ */
+int psdm_engine_snapshot_quotients(psdm_engine* e, float dt, const float* p3, const float* p1, int32_t n, float* q);
 
 /*
  * Forward modelling only (the receiver output Rec_point of

@@ -295,6 +295,17 @@ int reset_state(psdm_engine* e, Shot* s) {
     return PSDM_OK;
 }
 
+// The division constants of a time step (psdm_engine::div_cache).
+const std::pair<int, std::vector<float>>& div_constants(psdm_engine* e, float dt) {
+    auto it = e->div_cache.find(dt);
+    if (it == e->div_cache.end()) {
+        float r = 0.f, lo = 0.f, hi = 0.f, tiny = 0.f;
+        const int ok = fast_div_exact(dt, &r, &lo, &hi, &tiny) ? 1 : 0;
+        it = e->div_cache.emplace(dt, std::make_pair(ok, std::vector<float>{r, lo, hi, tiny})).first;
+    }
+    return it->second;
+}
+
 // Allocate and initialise the state of a shot from a window model already in
 // device memory (d_vp, (ny, nx) column-major).
 int setup_shot(psdm_engine* e, const psdm_params* prm, int ny, int nx, float dd, float dt, const float* d_vp,
@@ -349,17 +360,12 @@ int setup_shot(psdm_engine* e, const psdm_params* prm, int ny, int nx, float dd,
             s->cf2[k] = (float)c2[k];
         }
     }
-    auto it = e->div_cache.find(dt);
-    if (it == e->div_cache.end()) {
-        float r = 0.f, lo = 0.f, hi = 0.f, tiny = 0.f;
-        const int ok = fast_div_exact(dt, &r, &lo, &hi, &tiny) ? 1 : 0;
-        it = e->div_cache.emplace(dt, std::make_pair(ok, std::vector<float>{r, lo, hi, tiny})).first;
-    }
-    s->fast_div = it->second.first;
-    s->inv_dt = it->second.second[0];
-    s->div_lo = it->second.second[1];
-    s->div_hi = it->second.second[2];
-    s->div_tiny = it->second.second[3];
+    const auto& div = div_constants(e, dt);
+    s->fast_div = div.first;
+    s->inv_dt = div.second[0];
+    s->div_lo = div.second[1];
+    s->div_hi = div.second[2];
+    s->div_tiny = div.second[3];
 
     CUDA_TRY(cudaMemcpyAsync(s->fA, fA.data(), g.dn * sizeof(float), cudaMemcpyHostToDevice, e->stream));
     CUDA_TRY(cudaMemcpyAsync(s->fB, fB.data(), g.dn * sizeof(float), cudaMemcpyHostToDevice, e->stream));
@@ -3473,20 +3479,32 @@ int psdm_engine_dt_quotients(psdm_engine* e, float dt, const float* x, int32_t n
     TRY(check_engine(e));
     if (!x || !q || n <= 0 || n % 4) return fail(PSDM_ERR_ARG, "null argument, or n not a positive multiple of 4");
     TRY(sync(e));
-    auto it = e->div_cache.find(dt);
-    if (it == e->div_cache.end()) {
-        float r = 0.f, lo = 0.f, hi = 0.f, tiny = 0.f;
-        const int ok = fast_div_exact(dt, &r, &lo, &hi, &tiny) ? 1 : 0;
-        it = e->div_cache.emplace(dt, std::make_pair(ok, std::vector<float>{r, lo, hi, tiny})).first;
-    }
-    const std::vector<float>& c = it->second.second;
+    const auto& c = div_constants(e, dt);
     float *d_x = nullptr, *d_q = nullptr;
     TRY(e->get("dq_x", (size_t)n, &d_x));
     TRY(e->get("dq_q", (size_t)2 * n, &d_q));
     CUDA_TRY(cudaMemcpyAsync(d_x, x, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, e->stream));
-    const int rc = launch_dt_quotients(dt, c[0], c[1], c[2], it->second.first, d_x, d_q, n, e->stream);
+    const int rc = launch_dt_quotients(dt, c.second[0], c.second[1], c.second[2], c.first, d_x, d_q, n, e->stream);
     if (rc) return fail(PSDM_ERR_CUDA, "quotient launch: %s", cudaGetErrorString((cudaError_t)rc));
     CUDA_TRY(cudaMemcpyAsync(q, d_q, (size_t)2 * n * sizeof(float), cudaMemcpyDeviceToHost, e->stream));
+    return sync(e);
+}
+
+int psdm_engine_snapshot_quotients(psdm_engine* e, float dt, const float* p3, const float* p1, int32_t n, float* q) {
+    TRY(check_engine(e));
+    if (!p3 || !p1 || !q || n <= 0 || n % 4)
+        return fail(PSDM_ERR_ARG, "null argument, or n not a positive multiple of 4");
+    TRY(sync(e));
+    const auto& c = div_constants(e, dt);
+    float *d_p = nullptr, *d_q = nullptr;
+    TRY(e->get("dq_x", (size_t)2 * n, &d_p));
+    TRY(e->get("dq_q", (size_t)n, &d_q));
+    CUDA_TRY(cudaMemcpyAsync(d_p, p3, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, e->stream));
+    CUDA_TRY(cudaMemcpyAsync(d_p + n, p1, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, e->stream));
+    const int rc = launch_snapshot_quotients(dt, c.second[0], c.first, c.second[1], c.second[2], d_p, d_p + n, d_q, n,
+                                             e->stream);
+    if (rc) return fail(PSDM_ERR_CUDA, "quotient launch: %s", cudaGetErrorString((cudaError_t)rc));
+    CUDA_TRY(cudaMemcpyAsync(q, d_q, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, e->stream));
     return sync(e);
 }
 

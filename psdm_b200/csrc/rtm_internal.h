@@ -551,6 +551,10 @@ size_t region_max_floats();  // dynamic shared floats of a block (0 on failure)
 // img: the image of a plain backward pass stays in shared memory.
 int launch_regions(int mode, bool img, int pitch, const RegParams& rp, int nblocks, size_t floats, void* stream);
 
+// Snapshots of levels p3 and p1 as the region form makes them (n a multiple of 4).
+int launch_snapshot_quotients(float dt, float inv_dt, int fast_div, float div_lo, float div_hi, const float* p3,
+                              const float* p1, float* q, int n, void* stream);
+
 // One kernel whose bounded copy wait runs out (nothing is copied); sets *err.
 int launch_wait_timeout_probe(int* err, void* stream);
 int launch_dt_quotients(float dt, float inv_dt, float div_lo, float div_hi, int fast_div, const float* x, float* q,

@@ -133,29 +133,31 @@ __device__ __forceinline__ void fast_deriv2(const Consts& k, const float4& zm, c
 }
 
 // (p3 - p1) * 0.5 / dt of one float4, correctly rounded as div_dt does.  The
-// halved differences are scaled by 2^64, so that the reciprocal with its FMA
+// halved differences are scaled by -2^64, so that the reciprocal with its FMA
 // correction (q1) is exact for every nonzero one, and the quotients scaled
-// back with one rounding.  A quotient half way between two subnormals (diff =
-// half a step) takes the sign of q1's exact residual; an overflow of the
-// scaled form (diff is NaN) takes div_dt.  Testing for small differences
-// (below 2^-90) instead sent a band of about 20 cells ahead of the wavefront
-// through div_dt, and that set the pace of the whole pass.  A zero's sign is
-// not kept.
+// back with one rounding.  The residual is taken with its sign turned (q0 dt
+// - x), so that the correction of a zero is -0 and the zero keeps its sign (a
+// halved difference of the smallest subnormal rounds to one).  A quotient half
+// way between two subnormals (diff = half a step) takes the sign of q1's exact
+// residual; an overflow of the scaled form (diff is NaN) takes div_dt.  Testing
+// for small differences (below 2^-90) instead sent a band of about 20 cells
+// ahead of the wavefront through div_dt, and that set the pace of the whole
+// pass.
 __device__ __forceinline__ float4 snapshot4(const StepArgs& a, const Consts& kc, const float4& out, const float4& pm) {
-    const float2 half = make_float2(0.5f, 0.5f), up = make_float2(0x1p64f, 0x1p64f),
+    const float2 half = make_float2(0.5f, 0.5f), nup = make_float2(-0x1p64f, -0x1p64f),
                  dn = make_float2(0x1p-64f, 0x1p-64f);
-    const float2 r = make_float2(a.inv_dt, a.inv_dt), md = make_float2(-a.dt, -a.dt);
-    float2 h[2], q[2], q1[2], xs[2], diff[2];
+    const float2 nr = make_float2(-a.inv_dt, -a.inv_dt), dt = make_float2(a.dt, a.dt);
+    float2 h[2], q[2], q1[2], nx[2], diff[2];
     h[0] = __fmul2_rn(sub_p(kc, lo2(out), lo2(pm)), half);
     h[1] = __fmul2_rn(sub_p(kc, hi2(out), hi2(pm)), half);
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-        xs[k] = __fmul2_rn(h[k], up);
-        const float2 q0 = __fmul2_rn(xs[k], r);
-        const float2 e = __ffma2_rn(q0, md, xs[k]);
-        q1[k] = __ffma2_rn(e, r, q0);
+        nx[k] = __fmul2_rn(h[k], nup);
+        const float2 q0 = __fmul2_rn(nx[k], nr);
+        const float2 e = __ffma2_rn(q0, dt, nx[k]);
+        q1[k] = __ffma2_rn(e, nr, q0);
         q[k] = __fmul2_rn(q1[k], dn);
-        diff[k] = __ffma2_rn(q[k], make_float2(-0x1p64f, -0x1p64f), q1[k]);  // exact
+        diff[k] = __ffma2_rn(q[k], nup, q1[k]);  // exact
     }
     const float tie = 0x1p-86f;  // half a subnormal step
     const bool rare = !(fabsf(diff[0].x) < tie && fabsf(diff[0].y) < tie && fabsf(diff[1].x) < tie &&
@@ -167,11 +169,11 @@ __device__ __forceinline__ float4 snapshot4(const StepArgs& a, const Consts& kc,
         float v[4] = {q[0].x, q[0].y, q[1].x, q[1].y};
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-            const float2 e = __ffma2_rn(q1[k], md, xs[k]);  // sign of (true - q1)
+            const float2 e = __ffma2_rn(q1[k], dt, nx[k]);  // sign of (q1 - true)
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
                 const float ej = j == 0 ? e.x : e.y, dj = d[2 * k + j];
-                if (fabsf(dj) == tie && ej != 0.f && signbit(ej) == signbit(dj))
+                if (fabsf(dj) == tie && ej != 0.f && signbit(ej) != signbit(dj))
                     v[2 * k + j] = __fadd_rn(v[2 * k + j], copysignf(0x1p-149f, dj));
             }
         }
@@ -1482,7 +1484,33 @@ int launch_regions_p(int mode, bool img, const RegParams& rp, int nblocks, size_
     return launch_regions_t<2, false, P>(rp, nblocks, floats, st);
 }
 
+// The snapshots that snapshot4 makes of levels p3 and p1, n cells, n a
+// multiple of 4.
+__global__ void snapshot_quotients_kernel(const StepArgs a, float neg0, const float* p3, const float* p1, float* q,
+                                          int n) {
+    const int i = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+    if (i >= n) return;
+    Consts kc{};
+    kc.n0 = make_float2(neg0, neg0);
+    kc.m1 = make_float2(-1.f, -1.f);
+    *reinterpret_cast<float4*>(q + i) = snapshot4(a, kc, *reinterpret_cast<const float4*>(p3 + i),
+                                                  *reinterpret_cast<const float4*>(p1 + i));
+}
+
 }  // namespace
+
+int launch_snapshot_quotients(float dt, float inv_dt, int fast_div, float div_lo, float div_hi, const float* p3,
+                              const float* p1, float* q, int n, void* stream) {
+    if (n <= 0 || n % 4) return (int)cudaErrorInvalidValue;
+    StepArgs a{};
+    a.dt = dt;
+    a.inv_dt = inv_dt;
+    a.fast_div = fast_div;
+    a.div_lo = div_lo;
+    a.div_hi = div_hi;
+    snapshot_quotients_kernel<<<(n / 4 + 127) / 128, 128, 0, (cudaStream_t)stream>>>(a, -0.0f, p3, p1, q, n);
+    return (int)cudaGetLastError();
+}
 
 size_t region_max_floats() {
     static std::mutex lock;

@@ -256,6 +256,15 @@ class Engine:
         L.check(L.lib().psdm_engine_dt_quotients(self._h, float(dt), x, int(x.size), q))
         return q[:x.size], q[x.size:]
 
+    def snapshot_quotients(self, dt: float, p3, p1):
+        """psdm_engine_snapshot_quotients: (p3 - p1) * 0.5 / dt as the region launches store it, float32."""
+        p3, p1 = (np.ascontiguousarray(a, dtype=np.float32) for a in (p3, p1))
+        assert p3.shape == p1.shape
+        q = np.zeros(p3.size, dtype=np.float32)
+        L.check(L.lib().psdm_engine_snapshot_quotients(self._h, float(dt), p3.reshape(-1), p1.reshape(-1),
+                                                       int(p3.size), q))
+        return q.reshape(p3.shape)
+
     def batch_slots(self) -> int:
         return int(L.lib().psdm_engine_batch_slots(self._h))
 

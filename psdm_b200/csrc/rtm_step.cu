@@ -1281,10 +1281,17 @@ __global__ void quantize_many_kernel(const float* src, const unsigned int* amax,
 int launch_quantize_many(const float* src, const unsigned int* amax, void* dst, float* iscale, int n, int kind16,
                          int count, void* stream) {
     if (n <= 0 || count <= 0) return 0;
-    const dim3 grid(min((n / 4 + NT - 1) / NT, 148), count);
-    quantize_many_kernel<<<grid, dim3(32, NWARP), 0, (cudaStream_t)stream>>>(
-        src, amax, static_cast<unsigned short*>(dst), iscale, n, kind16);
-    return (int)cudaGetLastError();
+    constexpr int kMost = 65535;  // rows of a grid
+    unsigned short* d16 = static_cast<unsigned short*>(dst);
+    for (int m = 0; m < count; m += kMost) {
+        const dim3 grid(min((n / 4 + NT - 1) / NT, 148), min(count - m, kMost));
+        const size_t at = (size_t)m * n;
+        quantize_many_kernel<<<grid, dim3(32, NWARP), 0, (cudaStream_t)stream>>>(src + at, amax + m, d16 + at,
+                                                                                 iscale + m, n, kind16);
+        const cudaError_t rc = cudaGetLastError();
+        if (rc != cudaSuccess) return (int)rc;
+    }
+    return 0;
 }
 
 template <int FIXED>

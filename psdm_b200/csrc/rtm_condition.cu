@@ -146,12 +146,14 @@ int launch_condition(const CondArgs& c, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     // The cubics are shared where a trace's fit (6 floats a sample, up to 96 KB,
     // so that two blocks share a multiprocessor) and there are several samples
-    // an interval to share them.
+    // an interval to share them.  The kernel's limit belongs to the device, for
+    // every engine and thread: it is always set to the same 96 KB.
+    constexpr size_t kMost = 96 * 1024;
     const size_t bytes = (size_t)c.nt_data * sizeof(float4) + (2 * (size_t)c.nt_data + 3) * sizeof(float);
-    if (c.resample && c.nt_data >= 3 && bytes <= 96 * 1024 && c.nt_prop2 >= c.nt_data) {
+    if (c.resample && c.nt_data >= 3 && bytes <= kMost && c.nt_prop2 >= c.nt_data) {
         if (bytes > 48 * 1024) {
-            const cudaError_t rc = cudaFuncSetAttribute(condition_kernel<true>,
-                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+            const cudaError_t rc =
+                cudaFuncSetAttribute(condition_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost);
             if (rc != cudaSuccess) return (int)rc;
         }
         condition_kernel<true><<<c.nrec, 256, bytes, st>>>(c);

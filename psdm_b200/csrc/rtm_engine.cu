@@ -466,6 +466,66 @@ void set_buffers(const Shot& s, int it, StepArgs* a) {
     a->side_pm = s.side[c ^ 1];
 }
 
+// ---- launches whose blocks wait for one another --------------------------------
+
+// Cooperative launches of one device run side by side only while all their
+// blocks fit it together: a block waits for its neighbours, so two launches
+// that each hold part of the device would wait for good.  Kept per process,
+// whatever the engine, stream or thread.  Small windows need few blocks (24 for
+// 36 x 59 cells, 58 for 120 x 164), so several engines' passes overlap.
+struct CoopOrder {
+    std::mutex m;
+    struct Device {
+        CoopLedger ledger;
+        std::vector<cudaEvent_t> events;  // by id of the ledger
+    };
+    std::map<int, Device> devices;
+};
+CoopOrder& coop_order() {
+    static CoopOrder* o = new CoopOrder;  // outlives every engine
+    return *o;
+}
+
+// Run `launch` (a cooperative launch of `blocks` blocks on the engine's
+// stream, returning a CUDA error) in that order.
+template <class F>
+int coop_launch(psdm_engine* e, int blocks, const char* what, const F& launch) {
+    CoopOrder& o = coop_order();
+    std::lock_guard<std::mutex> lock(o.m);
+    CoopOrder::Device& d = o.devices[e->device];
+    d.ledger.prune([&](int id) { return cudaEventQuery(d.events[id]) == cudaSuccess; });
+    cudaGetLastError();  // "not ready" is no error of the launch below
+    const std::vector<int> follow = d.ledger.before(e->stream, blocks, e->num_sms);
+    for (int id : follow) CUDA_TRY(cudaStreamWaitEvent(e->stream, d.events[id], 0));
+    const int id = d.ledger.new_id();
+    int rc = PSDM_OK;
+    if (id == (int)d.events.size()) {
+        cudaEvent_t ev = nullptr;
+        const cudaError_t ce = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+        if (ce == cudaSuccess)
+            d.events.push_back(ev);
+        else
+            rc = fail(PSDM_ERR_CUDA, "cudaEventCreate: %s", cudaGetErrorString(ce));
+        if (rc != PSDM_OK) {
+            --d.ledger.ids;
+            return rc;
+        }
+    }
+    if (const int le = launch()) rc = fail(PSDM_ERR_CUDA, "%s launch: %s", what, cudaGetErrorString((cudaError_t)le));
+    if (rc == PSDM_OK) {
+        const cudaError_t re = cudaEventRecord(d.events[id], e->stream);
+        if (re != cudaSuccess) {  // it cannot be followed: let it end
+            cudaStreamSynchronize(e->stream);
+            rc = fail(PSDM_ERR_CUDA, "cudaEventRecord: %s", cudaGetErrorString(re));
+        }
+    }
+    if (rc == PSDM_OK)
+        d.ledger.queued(follow, id, e->stream, blocks);
+    else
+        d.ledger.idle.push_back(id);
+    return rc;
+}
+
 // The steps of a pass as the pass kernel's input: the arguments of the first
 // two steps as parity bases, and the values that change from step to step.
 // False when steps differ in anything else, or when a step reduces over the
@@ -583,9 +643,8 @@ int launch_pass_form(psdm_engine* e, int mode, const std::vector<StepArgs>& args
     pp.flags = d_flags;
     pp.abort = d_flags + ntiles;
     pp.err = a.err;
-    const int rc = launch_pass(mode, pp, grid, e->stream);
-    if (rc) return fail(PSDM_ERR_CUDA, "pass launch: %s", cudaGetErrorString((cudaError_t)rc));
-    return PSDM_OK;
+    // several blocks a multiprocessor: the whole device
+    return coop_launch(e, e->num_sms, "pass", [&] { return launch_pass(mode, pp, grid, e->stream); });
 }
 
 // One resident launch (res_kernel) for the whole pass: forward and plain
@@ -682,9 +741,7 @@ int launch_resident_form(psdm_engine* e, int mode, const std::vector<StepArgs>& 
     rp.flags = d_flags;
     rp.abort = d_flags + nreg;
     rp.err = a.err;
-    const int rc = launch_resident(mode, rp, e->stream);
-    if (rc) return fail(PSDM_ERR_CUDA, "resident pass launch: %s", cudaGetErrorString((cudaError_t)rc));
-    return PSDM_OK;
+    return coop_launch(e, e->num_sms, "resident pass", [&] { return launch_resident(mode, rp, e->stream); });
 }
 
 // Launch the step kernels of one pass.  The launches are captured once into
@@ -744,19 +801,6 @@ int launch_steps(psdm_engine* e, int mode, const std::vector<StepArgs>& args, in
 }
 
 // ---- passes as region launches (rtm_region.cu) --------------------------------
-
-// Cooperative launches of one device follow each other: a block of a region
-// launch waits for its neighbours, so two of them that each hold part of the
-// device would wait for good.  Every region launch of the process waits for
-// the device's previous one, whatever its engine, stream or thread.
-struct CoopOrder {
-    std::mutex m;
-    std::map<int, cudaEvent_t> done;
-};
-CoopOrder& coop_order() {
-    static CoopOrder* o = new CoopOrder;  // outlives every engine
-    return *o;
-}
 
 // The plan of a grid for `regions` blocks, made and uploaded on first use.
 // *out = null if the grid does not fit.  The pointer holds for the next
@@ -926,15 +970,9 @@ int region_launch(psdm_engine* e, int mode, RegPass& P, const std::vector<std::p
     TRY(e->get("reg_abort", 1, &rp.abort));
     CUDA_TRY(cudaMemsetAsync(rp.abort, 0, sizeof(int), e->stream));
     const bool img = mode == 1 && P.floats_img <= region_max_floats();
-    CoopOrder& o = coop_order();
-    std::lock_guard<std::mutex> lock(o.m);
-    cudaEvent_t& done = o.done[e->device];
-    if (done == nullptr) CUDA_TRY(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
-    CUDA_TRY(cudaStreamWaitEvent(e->stream, done, 0));
-    const int rc =
-        launch_regions(mode, img, P.pitch, rp, P.nblocks, img ? P.floats_img : P.floats, e->stream);
-    if (rc) return fail(PSDM_ERR_CUDA, "region launch: %s", cudaGetErrorString((cudaError_t)rc));
-    CUDA_TRY(cudaEventRecord(done, e->stream));
+    TRY(coop_launch(e, P.nblocks, "region", [&] {
+        return launch_regions(mode, img, P.pitch, rp, P.nblocks, img ? P.floats_img : P.floats, e->stream);
+    }));
     e->launches += 1;
     return PSDM_OK;
 }

@@ -535,6 +535,78 @@ struct KeyedSlots {
     }
     void drop(int i) { taken[i] = 0; }
 };
+// Launches of a device whose blocks wait for one another, a block a
+// multiprocessor at most.  Those that may run side by side hold at most `cap`
+// blocks together, so each gets all of its own: a launch follows its stream's
+// last one, and others until the rest leaves room, and takes their place.
+struct CoopLedger {
+    struct Flight {
+        int id, blocks;  // what the next launch waits for
+        const void* stream;
+        std::vector<int> followed;  // until all of these are done,
+        int until;                  // the blocks that they may hold
+        int weight() const { return until > blocks ? until : blocks; }
+    };
+    std::vector<Flight> flights;  // oldest first, weights at most `cap` in all
+    std::vector<int> idle;        // ids free for use again
+    int ids = 0;
+    // Drop what is done (completed(id) of a flight and what it followed).
+    template <class F>
+    void prune(const F& completed) {
+        for (size_t i = 0; i < flights.size();) {
+            Flight& f = flights[i];
+            const bool all = completed(f.id);
+            for (size_t k = 0; k < f.followed.size();)
+                if (all || completed(f.followed[k])) {
+                    idle.push_back(f.followed[k]);
+                    f.followed.erase(f.followed.begin() + (long)k);
+                } else {
+                    ++k;
+                }
+            if (f.followed.empty()) f.until = 0;
+            if (all) idle.push_back(f.id);
+            if (all)
+                flights.erase(flights.begin() + (long)i);
+            else
+                ++i;
+        }
+    }
+    int new_id() {
+        if (idle.empty()) return ids++;
+        const int id = idle.back();
+        idle.pop_back();
+        return id;
+    }
+    // The flights that a launch of `blocks` on `stream` follows: its stream's
+    // own, and the oldest ones until the others leave room.
+    std::vector<int> before(const void* stream, int blocks, int cap) const {
+        int others = 0;
+        for (const Flight& f : flights) others += f.stream == stream ? 0 : f.weight();
+        std::vector<int> w;
+        for (const Flight& f : flights) {
+            const bool own = f.stream == stream, more = !own && others + blocks > cap;
+            if (more) others -= f.weight();
+            if (own || more) w.push_back(f.id);
+        }
+        return w;
+    }
+    // That launch is queued as `id`.
+    void queued(const std::vector<int>& followed, int id, const void* stream, int blocks) {
+        Flight n{id, blocks, stream, followed, 0};
+        for (size_t i = 0, k = 0; i < flights.size();) {
+            const Flight& f = flights[i];
+            if (k < followed.size() && f.id == followed[k]) {  // in the order of `flights`
+                n.until += f.weight();
+                idle.insert(idle.end(), f.followed.begin(), f.followed.end());  // done before f is
+                flights.erase(flights.begin() + (long)i);
+                ++k;
+            } else {
+                ++i;
+            }
+        }
+        flights.push_back(n);
+    }
+};
 // Regions and packets of a padded grid for at most max_regions blocks of
 // max_floats shared floats, with columns of `pitch` (0: the cheaper one).
 // False if the grid does not fit.

@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <cstring>
 #include <array>
+#include <chrono>
 #include <complex>
 #include <map>
 #include <mutex>
@@ -117,7 +118,11 @@ struct psdm_engine {
     static constexpr int kRegPlans = 2 * kMaxSlots;
     RegSlot reg_plans[kRegPlans];
     KeyedSlots<std::array<int, 6>, kRegPlans> reg_keys;
-    std::map<std::array<int, 5>, double> reg_cost;  // region_step_cost by (ny, nx, dPML, fs, regions)
+    struct RegCost {
+        double step;  // estimated cycles, < 0: does not fit
+        int blocks;
+    };
+    std::map<std::array<int, 5>, RegCost> reg_cost;  // region_step_cost by (ny, nx, dPML, fs, regions)
     std::map<std::string, cudaEvent_t> reg_staged;  // copies out of a staging buffer done
     unsigned int reg_epoch = 1;  // tag of the next region launch's first step
     void* reg_board = nullptr;   // the board whose tags reg_epoch counts
@@ -474,12 +479,20 @@ void set_buffers(const Shot& s, int it, StepArgs* a) {
 // whatever the engine, stream or thread.  Small windows need few blocks (24 for
 // 36 x 59 cells, 58 for 120 x 164), so several engines' passes overlap.
 struct CoopOrder {
+    using Clock = std::chrono::steady_clock;
     std::mutex m;
     struct Device {
         CoopLedger ledger;
         std::vector<cudaEvent_t> events;  // by id of the ledger
+        int met = 1;                      // streams that had launches at once, the most
+        Clock::time_point when;           // of the last 50 to 100 ms
     };
     std::map<int, Device> devices;
+    int met(int device) {
+        std::lock_guard<std::mutex> lock(m);
+        const Device& d = devices[device];
+        return Clock::now() - d.when < std::chrono::milliseconds(100) ? d.met : 1;
+    }
 };
 CoopOrder& coop_order() {
     static CoopOrder* o = new CoopOrder;  // outlives every engine
@@ -495,8 +508,14 @@ int coop_launch(psdm_engine* e, int blocks, const char* what, const F& launch) {
     CoopOrder::Device& d = o.devices[e->device];
     d.ledger.prune([&](int id) { return cudaEventQuery(d.events[id]) == cudaSuccess; });
     cudaGetLastError();  // "not ready" is no error of the launch below
-    const std::vector<int> follow = d.ledger.before(e->stream, blocks, e->num_sms);
-    for (int id : follow) CUDA_TRY(cudaStreamWaitEvent(e->stream, d.events[id], 0));
+    const int met = 1 + d.ledger.others(e->stream);
+    const auto now = CoopOrder::Clock::now();
+    if (met >= d.met || now - d.when > std::chrono::milliseconds(50)) {
+        d.met = met;
+        d.when = now;
+    }
+    const std::vector<CoopLedger::Ref> follow = d.ledger.before(e->stream, blocks, e->num_sms);
+    for (const CoopLedger::Ref& f : follow) CUDA_TRY(cudaStreamWaitEvent(e->stream, d.events[f.id], 0));
     const int id = d.ledger.new_id();
     int rc = PSDM_OK;
     if (id == (int)d.events.size()) {
@@ -837,6 +856,46 @@ int region_plan(psdm_engine* e, const Grid& g, int fs, int regions, int pitch, p
     r.fits = true;
     *out = &r;
     return PSDM_OK;
+}
+
+// Estimated step of a grid on `regions` multiprocessors.
+const psdm_engine::RegCost& step_cost(psdm_engine* e, const Grid& g, int fs, int regions) {
+    const std::array<int, 5> key = {g.ny, g.nx, g.dPML, fs, regions};
+    auto it = e->reg_cost.find(key);
+    if (it == e->reg_cost.end()) {
+        if (e->reg_cost.size() > 256) e->reg_cost.clear();
+        psdm_engine::RegCost c{};
+        c.step = region_step_cost(g, fs, regions, region_max_floats(), &c.blocks);
+        it = e->reg_cost.emplace(key, c).first;
+    }
+    return it->second;
+}
+
+// Multiprocessors for one shot's passes: all of them, or a half or a quarter
+// where other engines' passes were met on the device lately, so that they run
+// side by side: a smaller share is taken where it is estimated to end as many
+// shots as there are engines in 0.7 of the time (the estimate is not exact, and
+// a pass that meets one on the whole device waits for it).  Shots/s of eight
+// engines in threads, every pass planned for the whole device against shares:
+// 120 x 164 window 479 against 550-700, 200 x 252 151 against 184-262, 331 x 324
+// 303 against 288-323, 700 x 744 274 and no share; eighths make 36 x 59 slower
+// (24 blocks are enough there: 4300 against 2880).
+int pass_regions(psdm_engine* e, const Grid& g, int fs) {
+    const int met = coop_order().met(e->device);
+    int best = e->num_sms;
+    if (met <= 1) return best;
+    double least = -1;
+    for (int k = 1; k <= met && k <= 4; k *= 2) {
+        const psdm_engine::RegCost c = step_cost(e, g, fs, e->num_sms / k);
+        if (c.step < 0) break;
+        const int side = std::max(1, e->num_sms / std::max(c.blocks, 1));
+        const double t = c.step * ((met + side - 1) / side);
+        if (least < 0 || t < 0.7 * least) {
+            least = t;
+            best = e->num_sms / k;
+        }
+    }
+    return best;
 }
 
 bool regions_on(const psdm_engine* e) {
@@ -1300,7 +1359,7 @@ int region_forward(psdm_engine* e, Shot& s, int nt, int store_snap, const float*
                    int nslots, int nrec, const int* h_rec_cell, float* d_rec) {
     std::vector<RegSpec> specs(1);
     specs[0].s = &s;
-    TRY(region_plan(e, s.g, s.fs, e->num_sms, 0, &specs[0].plan));
+    TRY(region_plan(e, s.g, s.fs, pass_regions(e, s.g, s.fs), 0, &specs[0].plan));
     if (!specs[0].plan) return 1;
     TRY(forward_spec(s, nt, store_snap, d_S, zs, xs, d_fields, nslots, nrec, h_rec_cell, d_rec, &specs[0]));
     RegPass P;
@@ -1458,7 +1517,7 @@ int region_backward(psdm_engine* e, Shot& s, int nt, int store_snap, int nt_snap
                     const float* h_w, float* d_image) {
     std::vector<RegSpec> specs(1);
     specs[0].s = &s;
-    TRY(region_plan(e, s.g, s.fs, e->num_sms, 0, &specs[0].plan));
+    TRY(region_plan(e, s.g, s.fs, pass_regions(e, s.g, s.fs), 0, &specs[0].plan));
     if (!specs[0].plan) return 1;
     TRY(backward_spec(s, nt, store_snap, nt_snap, d_back, reverse, nrec, zr, xr, d_fields, slot_lo, slot_hi, h_w,
                       d_image, &specs[0]));
@@ -1798,7 +1857,7 @@ int region_shot_checkpointed(psdm_engine* e, Shot& f, Shot& b, int NumRec, const
     std::vector<RegSpec> fw(1), re(1), bw(1);
     fw[0].s = re[0].s = &f;
     bw[0].s = &b;
-    TRY(region_plan(e, f.g, f.fs, e->num_sms, 0, &fw[0].plan));
+    TRY(region_plan(e, f.g, f.fs, pass_regions(e, f.g, f.fs), 0, &fw[0].plan));
     if (!fw[0].plan) return 1;
     re[0].plan = bw[0].plan = fw[0].plan;
     TRY(forward_spec(f, nt_prop2, store_snap, d_S, w.zs, w.xs, nullptr, 0, 0, nullptr, nullptr, &fw[0]));
@@ -2053,7 +2112,7 @@ int region_mixed_shot(psdm_engine* e, Shot& s, const MixedBufs& mb, int NumRec, 
                       const float* d_tgt, int store_snap, int nt_prop2, int nt_taper, const float* wts, float* d_imgp) {
     std::vector<RegSpec> fw(1), bw(1);
     fw[0].s = bw[0].s = &s;
-    TRY(region_plan(e, s.g, s.fs, e->num_sms, 0, &fw[0].plan));
+    TRY(region_plan(e, s.g, s.fs, pass_regions(e, s.g, s.fs), 0, &fw[0].plan));
     if (!fw[0].plan) return 1;
     bw[0].plan = fw[0].plan;
     float* stage = nullptr;
@@ -2583,17 +2642,6 @@ std::vector<int> batch_shares(const psdm_engine* e, const BatchJob& j, int first
     return r;
 }
 
-// Estimated step of a grid on `regions` multiprocessors; < 0 if it does not fit.
-double batch_step_cost(psdm_engine* e, const Grid& g, int fs, int regions) {
-    const std::array<int, 5> key = {g.ny, g.nx, g.dPML, fs, regions};
-    auto it = e->reg_cost.find(key);
-    if (it == e->reg_cost.end()) {
-        if (e->reg_cost.size() > 256) e->reg_cost.clear();
-        it = e->reg_cost.emplace(key, region_step_cost(g, fs, regions, region_max_floats())).first;
-    }
-    return it->second;
-}
-
 // Shots of the group that starts at `first`: the size with the least
 // estimated time a shot, of at most `most`; 0 if the first shot does not fit.
 int batch_group(psdm_engine* e, const BatchJob& j, int first, int most) {
@@ -2604,7 +2652,7 @@ int batch_group(psdm_engine* e, const BatchJob& j, int first, int most) {
         double t = 0;
         for (int k = 0; k < n && t >= 0; ++k) {
             const psdm_shot& sh = j.shots[first + k];
-            const double c = batch_step_cost(e, make_grid(j.prm->dPML, j.ny, sh.nx_w), j.prm->fs != 0, share[k]);
+            const double c = step_cost(e, make_grid(j.prm->dPML, j.ny, sh.nx_w), j.prm->fs != 0, share[k]).step;
             t = c < 0 ? -1.0 : std::max(t, c * ((double)sh.nt_prop2 + sh.nt_taper));
         }
         if (t < 0) {

@@ -540,10 +540,14 @@ struct KeyedSlots {
 // blocks together, so each gets all of its own: a launch follows its stream's
 // last one, and others until the rest leaves room, and takes their place.
 struct CoopLedger {
-    struct Flight {
-        int id, blocks;  // what the next launch waits for
+    struct Ref {
+        int id;  // what a launch that follows waits for
         const void* stream;
-        std::vector<int> followed;  // until all of these are done,
+    };
+    struct Flight {
+        Ref ref;
+        int blocks;
+        std::vector<Ref> followed;  // until all of these are done,
         int until;                  // the blocks that they may hold
         int weight() const { return until > blocks ? until : blocks; }
     };
@@ -555,16 +559,16 @@ struct CoopLedger {
     void prune(const F& completed) {
         for (size_t i = 0; i < flights.size();) {
             Flight& f = flights[i];
-            const bool all = completed(f.id);
+            const bool all = completed(f.ref.id);
             for (size_t k = 0; k < f.followed.size();)
-                if (all || completed(f.followed[k])) {
-                    idle.push_back(f.followed[k]);
+                if (all || completed(f.followed[k].id)) {
+                    idle.push_back(f.followed[k].id);
                     f.followed.erase(f.followed.begin() + (long)k);
                 } else {
                     ++k;
                 }
             if (f.followed.empty()) f.until = 0;
-            if (all) idle.push_back(f.id);
+            if (all) idle.push_back(f.ref.id);
             if (all)
                 flights.erase(flights.begin() + (long)i);
             else
@@ -577,27 +581,41 @@ struct CoopLedger {
         idle.pop_back();
         return id;
     }
+    // Streams other than `stream` with launches that may not be done.
+    int others(const void* stream) const {
+        std::vector<const void*> seen = {stream};
+        auto see = [&seen](const Ref& r) {
+            for (const void* s : seen)
+                if (s == r.stream) return;
+            seen.push_back(r.stream);
+        };
+        for (const Flight& f : flights) {
+            see(f.ref);
+            for (const Ref& r : f.followed) see(r);
+        }
+        return (int)seen.size() - 1;
+    }
     // The flights that a launch of `blocks` on `stream` follows: its stream's
     // own, and the oldest ones until the others leave room.
-    std::vector<int> before(const void* stream, int blocks, int cap) const {
-        int others = 0;
-        for (const Flight& f : flights) others += f.stream == stream ? 0 : f.weight();
-        std::vector<int> w;
+    std::vector<Ref> before(const void* stream, int blocks, int cap) const {
+        int rest = 0;
+        for (const Flight& f : flights) rest += f.ref.stream == stream ? 0 : f.weight();
+        std::vector<Ref> w;
         for (const Flight& f : flights) {
-            const bool own = f.stream == stream, more = !own && others + blocks > cap;
-            if (more) others -= f.weight();
-            if (own || more) w.push_back(f.id);
+            const bool own = f.ref.stream == stream, more = !own && rest + blocks > cap;
+            if (more) rest -= f.weight();
+            if (own || more) w.push_back(f.ref);
         }
         return w;
     }
     // That launch is queued as `id`.
-    void queued(const std::vector<int>& followed, int id, const void* stream, int blocks) {
-        Flight n{id, blocks, stream, followed, 0};
+    void queued(const std::vector<Ref>& followed, int id, const void* stream, int blocks) {
+        Flight n{{id, stream}, blocks, followed, 0};
         for (size_t i = 0, k = 0; i < flights.size();) {
             const Flight& f = flights[i];
-            if (k < followed.size() && f.id == followed[k]) {  // in the order of `flights`
+            if (k < followed.size() && f.ref.id == followed[k].id) {  // in the order of `flights`
                 n.until += f.weight();
-                idle.insert(idle.end(), f.followed.begin(), f.followed.end());  // done before f is
+                for (const Ref& r : f.followed) idle.push_back(r.id);  // done before f is
                 flights.erase(flights.begin() + (long)i);
                 ++k;
             } else {
@@ -611,9 +629,9 @@ struct CoopLedger {
 // max_floats shared floats, with columns of `pitch` (0: the cheaper one).
 // False if the grid does not fit.
 bool plan_regions(const Grid& g, int fs, int max_regions, size_t max_floats, RegPlan* plan, int pitch = 0);
-// The estimated cycles of a step of that plan, without the plan; < 0 if the
-// grid does not fit.
-double region_step_cost(const Grid& g, int fs, int max_regions, size_t max_floats);
+// The estimated cycles of a step of that plan and its regions, without the
+// plan; < 0 if the grid does not fit.
+double region_step_cost(const Grid& g, int fs, int max_regions, size_t max_floats, int* blocks = nullptr);
 // The regions' shares of a pass: injection points (linear cells x * ldz +
 // device row of interior cells, with their trace) and receivers.  False if
 // the source buffers do not fit.

@@ -1255,11 +1255,18 @@ double best_cut(std::vector<Part>& parts, int max_regions, size_t max_floats, in
 
 }  // namespace
 
-double region_step_cost(const Grid& g, int fs, int max_regions, size_t max_floats) {
+double region_step_cost(const Grid& g, int fs, int max_regions, size_t max_floats, int* blocks) {
     std::vector<Part> parts;
     int P = 0;
     bool img = false;
-    return grid_parts(g, fs, max_regions, &parts) ? best_cut(parts, max_regions, max_floats, 0, &P, &img) : -1.0;
+    const double best = grid_parts(g, fs, max_regions, &parts)
+                            ? best_cut(parts, max_regions, max_floats, 0, &P, &img) : -1.0;
+    if (blocks != nullptr) {
+        *blocks = 0;
+        if (best >= 0)
+            for (Part& p : parts) *blocks += cut_part(&p, P, best, max_floats, max_regions, img);
+    }
+    return best;
 }
 
 bool plan_regions(const Grid& g, int fs, int max_regions, size_t max_floats, RegPlan* plan, int pitch) {

@@ -57,7 +57,7 @@ int main(int argc, char** argv) {
             l.prune([&](int id) { return all[newest[id]].state == 2; });
         Launch x{blocks, 0, {}};
         const auto follow = l.before(&place[st], blocks, cap);
-        for (int f : follow) x.after.push_back(newest[f]);
+        for (const auto& f : follow) x.after.push_back(newest[f.id]);
         if (last[st] >= 0) x.after.push_back(last[st]);
         const int id = l.new_id();
         l.queued(follow, id, &place[st], blocks);

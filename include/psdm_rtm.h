@@ -220,7 +220,7 @@ int psdm_engine_set_checkpointing(psdm_engine* e, int32_t interval);
 int psdm_engine_set_reconstruction(psdm_engine* e, int32_t on);
 /*
  * Launch form of one shot's passes (psdm_rtm_shot, psdm_model_shot and their
- * device variants).  Until it is set, every pass (plain, mixed-precision,
+ * device variants).  -1 (default): every pass (plain, mixed-precision,
  * checkpointed, and those of the batched calls, several shots side by side)
  * runs as one cooperative launch of one block per region of the grid where
  * the grid fits the device's shared memory (the interior, C-PML strips and
@@ -233,9 +233,9 @@ int psdm_engine_set_reconstruction(psdm_engine* e, int32_t on);
  * only the ring with its neighbours (grids that fit the device's blocks;
  * others fall back to one launch per step); 0 launches one kernel
  * per time step (replayed from a CUDA graph).  Same results bit for bit.
- * With a form set, passes with the mixed-precision snapshots use one launch
+ * With 0, 1 or 2, passes with the mixed-precision snapshots use one launch
  * per step.
- * Values other than 0, 1 and 2 return PSDM_ERR_ARG.
+ * Other values return PSDM_ERR_ARG.
  */
 int psdm_engine_set_pass_launch(psdm_engine* e, int32_t on);
 /*

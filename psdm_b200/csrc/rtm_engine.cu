@@ -102,7 +102,7 @@ struct psdm_engine {
     std::vector<int> res_key[2];   // resident form, by pass kind
     int res_nreg[2] = {0, 0}, res_sw[2] = {0, 0};
     cudaEvent_t pass_staged[3] = {nullptr, nullptr, nullptr};  // copies out of the staging buffers done
-    // Until a launch form is chosen (psdm_engine_set_pass_launch), passes run
+    // Unless a launch form is chosen (psdm_engine_set_pass_launch), passes run
     // as one region launch each where the grid fits (rtm_region.cu).
     bool use_regions = true;
     // Region plans by (ny, nx, dPML, fs, regions, pitch), each with its lists in
@@ -3374,9 +3374,9 @@ int psdm_engine_autotune(psdm_engine* e, const psdm_params* prm, int32_t ny, int
 
 int psdm_engine_set_pass_launch(psdm_engine* e, int32_t on) {
     TRY(check_engine(e));
-    if (on < 0 || on > 2) return fail(PSDM_ERR_ARG, "pass launch form must be 0, 1 or 2 (got %d)", on);
-    e->use_pass = on;
-    e->use_regions = false;
+    if (on < -1 || on > 2) return fail(PSDM_ERR_ARG, "pass launch form must be -1, 0, 1 or 2 (got %d)", on);
+    e->use_pass = std::max(on, 0);
+    e->use_regions = on == -1;
     return PSDM_OK;
 }
 

@@ -221,8 +221,8 @@ class Engine:
 
     def set_pass_launch(self, on):
         """psdm_engine_set_pass_launch: one launch per step (0 / False), one cooperative launch per pass
-        with tiles (1 / True) or with regions resident in shared memory (2); until it is called the
-        engine chooses (one launch per pass where the grid fits)."""
+        with tiles (1 / True) or with regions resident in shared memory (2); -1, the default, lets the
+        engine choose (one launch per pass where the grid fits)."""
         L.check(L.lib().psdm_engine_set_pass_launch(self._h, int(on)))
 
     def set_steps_per_launch(self, steps: int):

@@ -898,6 +898,14 @@ int pass_regions(psdm_engine* e, const Grid& g, int fs) {
     return best;
 }
 
+// Fewest steps for which a region launch is taken: it reads and writes the
+// whole state, so short ones are slower than launches of a step.  Checkpointed
+// shots (a launch a segment) broke even with segments of 2 steps on 36 x 59 and
+// 200 x 249 windows, 4 on 500 x 701, 6 on 700 x 901, 9 on 300 x 2774 and 14 on
+// 1200 x 1137 (segments of 1, 2, 5 and 10 steps there: 1.79, 1.64, 1.34 and 1.10
+// of the time of step launches; 20: 0.89); whole passes of so many steps alike.
+int region_min_steps(const Grid& g) { return 2 + (int)((double)g.nyt * g.nxt / 120000.0); }
+
 bool regions_on(const psdm_engine* e) {
     return e->use_regions && e->use_pass == 0 && e->steps_per_launch == 1 && region_max_floats() > 0;
 }
@@ -1359,6 +1367,7 @@ int region_forward(psdm_engine* e, Shot& s, int nt, int store_snap, const float*
                    int nslots, int nrec, const int* h_rec_cell, float* d_rec) {
     std::vector<RegSpec> specs(1);
     specs[0].s = &s;
+    if (nt - 1 < region_min_steps(s.g)) return 1;
     TRY(region_plan(e, s.g, s.fs, pass_regions(e, s.g, s.fs), 0, &specs[0].plan));
     if (!specs[0].plan) return 1;
     TRY(forward_spec(s, nt, store_snap, d_S, zs, xs, d_fields, nslots, nrec, h_rec_cell, d_rec, &specs[0]));
@@ -1517,6 +1526,7 @@ int region_backward(psdm_engine* e, Shot& s, int nt, int store_snap, int nt_snap
                     const float* h_w, float* d_image) {
     std::vector<RegSpec> specs(1);
     specs[0].s = &s;
+    if (nt - 1 < region_min_steps(s.g)) return 1;
     TRY(region_plan(e, s.g, s.fs, pass_regions(e, s.g, s.fs), 0, &specs[0].plan));
     if (!specs[0].plan) return 1;
     TRY(backward_spec(s, nt, store_snap, nt_snap, d_back, reverse, nrec, zr, xr, d_fields, slot_lo, slot_hi, h_w,
@@ -1710,10 +1720,12 @@ void mixed_backward_args(const MixedBufs& mb, int nt, const float* h_w, std::vec
 // 1136 window pauses every 384 steps at ks = 4, under 2 % of the pass.
 
 // Snapshots staged by one launch: `bytes` of staging, an eighth of the free
-// memory at most; 0 when there is no room for a few.
-int mixed_stage(psdm_engine* e, size_t fstride, int nsnap, size_t bytes, const std::string& tag, float** stage,
+// memory at most; 0 when there is no room for those of a launch that is worth
+// it (region_min_steps), or for a few.
+int mixed_stage(psdm_engine* e, const Grid& g, int ks, int nsnap, size_t bytes, const std::string& tag, float** stage,
                 int* nstage) {
     *nstage = 0;
+    const size_t fstride = g.field_cells();
     const size_t have = e->bufs[("reg_staging" + tag)].bytes;
     size_t room = have;
     // the driver is asked only where the buffer is to grow: the query took tens of milliseconds at times
@@ -1724,7 +1736,8 @@ int mixed_stage(psdm_engine* e, size_t fstride, int nsnap, size_t bytes, const s
         room = std::max(have, std::min(bytes, fr / 8));
     }
     const int n = (int)std::min<size_t>(room / (fstride * sizeof(float)), (size_t)std::max(nsnap, 1));
-    if (n < std::min(4, std::max(nsnap, 1))) return PSDM_OK;
+    const int few = std::max(4, (region_min_steps(g) + ks - 1) / ks);
+    if (n < std::min(few, std::max(nsnap, 1))) return PSDM_OK;
     TRY(e->get(("reg_staging" + tag).c_str(), fstride * (size_t)n, stage));
     *nstage = n;
     return PSDM_OK;
@@ -1857,6 +1870,7 @@ int region_shot_checkpointed(psdm_engine* e, Shot& f, Shot& b, int NumRec, const
     std::vector<RegSpec> fw(1), re(1), bw(1);
     fw[0].s = re[0].s = &f;
     bw[0].s = &b;
+    if (std::min(K, nsteps) < region_min_steps(f.g)) return 1;
     TRY(region_plan(e, f.g, f.fs, pass_regions(e, f.g, f.fs), 0, &fw[0].plan));
     if (!fw[0].plan) return 1;
     re[0].plan = bw[0].plan = fw[0].plan;
@@ -2112,12 +2126,13 @@ int region_mixed_shot(psdm_engine* e, Shot& s, const MixedBufs& mb, int NumRec, 
                       const float* d_tgt, int store_snap, int nt_prop2, int nt_taper, const float* wts, float* d_imgp) {
     std::vector<RegSpec> fw(1), bw(1);
     fw[0].s = bw[0].s = &s;
+    if (std::min(nt_prop2, nt_taper) - 1 < region_min_steps(s.g)) return 1;
     TRY(region_plan(e, s.g, s.fs, pass_regions(e, s.g, s.fs), 0, &fw[0].plan));
     if (!fw[0].plan) return 1;
     bw[0].plan = fw[0].plan;
     float* stage = nullptr;
     int nstage = 0;
-    TRY(mixed_stage(e, mb.fstride, mb.nsnap, (size_t)512 << 20, "", &stage, &nstage));
+    TRY(mixed_stage(e, s.g, mb.ks, mb.nsnap, (size_t)512 << 20, "", &stage, &nstage));
     if (nstage == 0) return 1;
     TRY(forward_spec(s, nt_prop2, store_snap, d_S, w.zs, w.xs, nullptr, 0, 0, nullptr, nullptr, &fw[0]));
     mixed_forward_vars(mb, stage, nstage, fw[0].var);
@@ -2696,7 +2711,7 @@ int batch_group_run(psdm_engine* e, const BatchJob& j, std::vector<BatchSlot>& s
         if (mixed) {
             TRY(mixed_bufs(e, sl.s, j.prm->precision, j.store_snap, sh.nt_prop2, sl.tag, &sl.mb));
             int ns = 0;
-            TRY(mixed_stage(e, fstride, nsnap, ((size_t)512 << 20) / n, sl.tag, &stage[k], &ns));
+            TRY(mixed_stage(e, g, j.store_snap, nsnap, ((size_t)512 << 20) / n, sl.tag, &stage[k], &ns));
             if (ns == 0) return 1;
             nstage = std::min(nstage, ns);
         } else if (nsnap > 0) {

@@ -3499,13 +3499,13 @@ static int designed_filter(psdm_engine* e, int nt, float dt, int typef, float f1
     const size_t hb = (size_t)(ts / 2 + 1) * sizeof(std::complex<double>);
     TRY(e->get(("filt_tw" + t).c_str(), (size_t)4 * M, &tw));
     TRY(e->get(("filt_G" + t).c_str(), (size_t)2 * (M + 1), &G));
-    TRY(e->get("filt_design", filter_design_bytes(ts, nt, M), &work));
+    TRY(e->get("filt_design", filter_design_bytes(ts, nt), &work));
     std::vector<std::complex<double>> H(ts / 2 + 1);
     butterworth_response_f64(ts, 1.f / dt, typef, f1, f2, H.data());
     CUDA_TRY(cudaMemcpyAsync(work, H.data(), hb, cudaMemcpyHostToDevice, e->stream));
     const int rc = design_filter(work, work + hb, ts, nt, M, tw, G, e->stream);
     if (rc) return fail(PSDM_ERR_CUDA, "filter design launch: %s", cudaGetErrorString((cudaError_t)rc));
-    e->launches += 5;
+    e->launches += 3;
     f.nt = nt;
     f.typef = typef;
     f.dt = dt;

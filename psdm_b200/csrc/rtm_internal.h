@@ -314,7 +314,7 @@ void butterworth_response(int ts, float fe, int typef, float f1, float fc, std::
 constexpr int kFilterMaxPoints = 16384;
 int filter_points(int nt);
 void butterworth_response_f64(int ts, float fe, int typef, float f1, float fc, std::complex<double>* H);
-size_t filter_design_bytes(int ts, int nt, int M);
+size_t filter_design_bytes(int ts, int nt);
 int design_filter(const void* d_H, void* work, int ts, int nt, int M, void* d_tw, void* d_G, void* stream);
 int launch_filter(float* d_tr, int nt, int num, int M, const void* d_tw, const void* d_G, void* stream);
 int make_fft_plans(int ts, int num, int* plans);  // plans[0] real-to-complex, plans[1] complex-to-real

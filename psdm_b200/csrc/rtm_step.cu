@@ -663,11 +663,10 @@ constexpr int smem_floats() {
 
 // One time step of one shot.
 //
-// MANY = false: about as many tiles as resident blocks (operands in L2).  The
-// step is latency: a block starts on the tile of its own number, so that the
-// counter is asked only for further ones (against asking it for the first
-// too: a shot of 3000 steps on a 200 x 249 window 54.0 -> 48.2 ms, of 2000 on
-// 1200 x 1136 40.8 -> 37.7).
+// MANY = false: no more tiles than resident blocks (launch_mode's rule; operands
+// in L2).  The step is latency: a block a tile, and the counter is not asked
+// (against asking it for each tile: a shot of 3000 steps on a 200 x 249 window
+// 54.0 -> 48.2 ms, of 2000 on 1200 x 1136 40.8 -> 37.7).
 //
 // MANY = true: several tiles a block (launch_mode's rule), operands beyond L2.
 // The step is bound by loads in flight and by what the tiles leave idle, so
@@ -697,7 +696,6 @@ __global__ void __launch_bounds__(NT, 5) step_kernel(const StepArgs a) {
     if (tid == 0) {
         mbar_init(&bar, 1);
         s_blk_amax = 0u;
-        if (!MANY) tile_id = blockIdx.x;
     }
     // Receivers of the previous step (p is that step's p3, read-only during
     // this step): spread over the blocks, a receiver per thread, loaded before
@@ -718,12 +716,12 @@ __global__ void __launch_bounds__(NT, 5) step_kernel(const StepArgs a) {
         }
     }
     if (MODE == 0 && a.q_src != nullptr) quantize_part(a.q_src, a.q_amax, a.q_dst, a.q_iscale, a.q_n, a.kind16, tid);
-    // Persistent blocks take tiles from this step's counter, in order (heaviest
-    // rect types first) or spread; the other counter is cleared for the next step.
+    // Persistent blocks (MANY) take tiles from this step's counter; the other
+    // counter is cleared for the next step.
     if (blockIdx.x == 0 && tid == 0) a.tile_counter[a.counter_sel ^ 1] = 0;
     __syncthreads();
     uint32_t phase = 0;
-    const int total = a.r_first[a.nrect], grid = gridDim.x;
+    const int total = a.r_first[a.nrect];
     int nin = 0;  // interior tiles, the first of the list
     if (MANY) {
         int r = 0;
@@ -732,16 +730,12 @@ __global__ void __launch_bounds__(NT, 5) step_kernel(const StepArgs a) {
     }
     const int nbd = total - nin, span = max(total / 2, nbd);  // nbd others among the first span tiles
     for (;;) {
-        if (MANY && tid == 0) tile_id = atomicAdd(a.tile_counter + a.counter_sel, 1);
-        __syncthreads();
-        int b = tile_id;
-        if (b >= total) {
-            if (MODE == 0 && tid == 0 && a.field_amax != nullptr && s_blk_amax != 0u)
-                atomicMax(a.field_amax, s_blk_amax);
-            if (MODE == 0 && rec_i >= 0) a.rec_out[(size_t)rec_i * a.rec_ld + a.rec_t] = rec_v;
-            return;
-        }
+        int b = blockIdx.x;
         if (MANY) {
+            if (tid == 0) tile_id = atomicAdd(a.tile_counter + a.counter_sel, 1);
+            __syncthreads();
+            b = tile_id;
+            if (b >= total) break;
             const int k0 = min(nbd, (int)((long long)b * nbd / span)),
                       k1 = min(nbd, (int)((long long)(b + 1) * nbd / span));
             b = k1 > k0 ? nin + k0 : b - k0;
@@ -764,10 +758,11 @@ __global__ void __launch_bounds__(NT, 5) step_kernel(const StepArgs a) {
             case 4: rowband_tile<MODE>(a, sm, r, t); break;
             default: generic_tile<MODE>(a, sm, r, t); break;
         }
-        __syncthreads();  // shared tile and tile_id are reused
-        if (!MANY && tid == 0)
-            tile_id = grid >= total ? total : grid + atomicAdd(a.tile_counter + a.counter_sel, 1);
+        __syncthreads();  // shared tile and tile_id are reused, s_blk_amax is read
+        if (!MANY) break;
     }
+    if (MODE == 0 && tid == 0 && a.field_amax != nullptr && s_blk_amax != 0u) atomicMax(a.field_amax, s_blk_amax);
+    if (MODE == 0 && rec_i >= 0) a.rec_out[(size_t)rec_i * a.rec_ld + a.rec_t] = rec_v;
 }
 
 // One tile (block-local index b of the step described by `a`).  Returns

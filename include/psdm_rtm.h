@@ -302,6 +302,13 @@ int32_t psdm_engine_batch_slots(const psdm_engine* e);
  * message when the path works; the engine stays usable afterwards.
  */
 int psdm_engine_check_wait_timeout(psdm_engine* e);
+/*
+ * The same for the region launches: a small pass is launched without its last
+ * region, so that the others wait for packets that nobody sends, give up after
+ * their time limit (about 2 s) and report.  Returns PSDM_ERR_CUDA with the
+ * pass kernels' timeout message when the path works; the engine stays usable.
+ */
+int psdm_engine_check_region_timeout(psdm_engine* e);
 
 /*
  * The snapshot quotient of the forward kernels, x / dt, for n host inputs (no

@@ -3576,6 +3576,36 @@ int psdm_engine_check_wait_timeout(psdm_engine* e) {
     return sync(e);
 }
 
+int psdm_engine_check_region_timeout(psdm_engine* e) {
+    TRY(check_engine(e));
+    TRY(sync(e));
+    // two steps of a small window without a source, its last region left out
+    psdm_params prm{};
+    prm.dPML = 8;
+    prm.strategy = 1;
+    prm.precision = PSDM_PREC_FP32;
+    const int ny = 36, nx = 48, nt = 3;
+    const std::vector<float> vp((size_t)ny * nx, 2000.f), S(nt, 0.f);
+    float *d_vp = nullptr, *d_S = nullptr;
+    TRY(e->get("probe_vp", vp.size(), &d_vp));
+    TRY(e->get("probe_S", S.size(), &d_S));
+    CUDA_TRY(cudaMemcpyAsync(d_vp, vp.data(), vp.size() * sizeof(float), cudaMemcpyHostToDevice, e->stream));
+    CUDA_TRY(cudaMemcpyAsync(d_S, S.data(), S.size() * sizeof(float), cudaMemcpyHostToDevice, e->stream));
+    Shot s;
+    TRY(setup_shot(e, &prm, ny, nx, 10.f, 1e-3f, d_vp, &s, "_probe"));
+    std::vector<RegSpec> specs(1);
+    specs[0].s = &s;
+    TRY(region_plan(e, s.g, s.fs, e->num_sms, 0, &specs[0].plan));
+    if (!specs[0].plan) return fail(PSDM_ERR_CUDA, "the region form has no plan for the probe's window");
+    TRY(forward_spec(s, nt, 1, d_S, s.g.dn + 1, s.g.dn + nx / 2, nullptr, 0, 0, nullptr, nullptr, &specs[0]));
+    RegPass P;
+    if (region_prepare(e, specs, "0", &P) != PSDM_OK)
+        return fail(PSDM_ERR_CUDA, "the region form cannot prepare the probe");
+    P.nblocks -= 1;
+    TRY(region_launch_all(e, 0, P));
+    return sync(e);
+}
+
 int psdm_engine_dt_quotients(psdm_engine* e, float dt, const float* x, int32_t n, float* q) {
     TRY(check_engine(e));
     if (!x || !q || n <= 0 || n % 4) return fail(PSDM_ERR_ARG, "null argument, or n not a positive multiple of 4");

@@ -52,11 +52,11 @@ inline Grid make_grid(int dPML, int ny, int nx) {
 // Message for a nonzero value of a step kernel's error word: 1 = a bounded
 // wait for the tile's shared-memory copies ran out, 2 = the tile plan was
 // made for another launch form, 3 = a pass kernel gave up waiting for its
-// neighbouring tiles.
+// neighbouring tiles or regions.
 inline const char* step_error_message(int code) {
     switch (code) {
         case 2: return "a step kernel was given a tile plan for another launch form";
-        case 3: return "a pass kernel timed out waiting for neighbouring tiles";
+        case 3: return "a pass kernel timed out waiting for neighbouring tiles or regions";
         default: return "a step kernel timed out waiting for its shared-memory copies";
     }
 }

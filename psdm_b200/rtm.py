@@ -249,6 +249,10 @@ class Engine:
         """psdm_engine_check_wait_timeout: raises PsdmError when the failure path works."""
         L.check(L.lib().psdm_engine_check_wait_timeout(self._h))
 
+    def check_region_timeout(self):
+        """psdm_engine_check_region_timeout: raises PsdmError when the failure path works."""
+        L.check(L.lib().psdm_engine_check_region_timeout(self._h))
+
     def dt_quotients(self, dt: float, x):
         """psdm_engine_dt_quotients: (the interior tiles' x / dt, the general form's x / dt), float32."""
         x = np.ascontiguousarray(x, dtype=np.float32)

@@ -1719,26 +1719,52 @@ void mixed_backward_args(const MixedBufs& mb, int nt, const float* h_w, std::vec
 // launch, and a conversion launch follows: with 512 MB of staging a 1200 x
 // 1136 window pauses every 384 steps at ks = 4, under 2 % of the pass.
 
-// Snapshots staged by one launch: `bytes` of staging, an eighth of the free
-// memory at most; 0 when there is no room for those of a launch that is worth
-// it (region_min_steps), or for a few.
-int mixed_stage(psdm_engine* e, const Grid& g, int ks, int nsnap, size_t bytes, const std::string& tag, float** stage,
-                int* nstage) {
+// A shot whose snapshots are staged.
+struct Staged {
+    Grid g;
+    int ks, nsnap;
+    float* stage = nullptr;
+};
+
+// Snapshots that each of the shots stages in one launch, in shares of one buffer
+// of `kStaging` bytes, an eighth of the free memory at most (inside what
+// psdm_plan_memory leaves free); 0 when there is no room for those of a launch
+// that is worth it (region_min_steps), or for a few.
+constexpr size_t kStaging = (size_t)512 << 20;
+int mixed_stage(psdm_engine* e, std::vector<Staged>& shots, int* nstage) {
     *nstage = 0;
-    const size_t fstride = g.field_cells();
-    const size_t have = e->bufs[("reg_staging" + tag)].bytes;
+    auto bytes = [&](int n) {
+        size_t b = 0;
+        for (const Staged& s : shots) b += s.g.field_cells() * sizeof(float) * (size_t)std::min(n, std::max(s.nsnap, 1));
+        return b;
+    };
+    int most = 1;
+    for (const Staged& s : shots) most = std::max(most, s.nsnap);
+    const size_t have = e->bufs["reg_staging"].bytes;
     size_t room = have;
     // the driver is asked only where the buffer is to grow: the query took tens of milliseconds at times
     // (8 FP16 shots of 1200 x 1136, 1200 steps: passes of 140-200 ms among those of 102)
-    if (have < std::min(bytes, fstride * sizeof(float) * (size_t)std::max(nsnap, 1))) {
+    if (have < std::min(kStaging, bytes(most))) {
         size_t fr = 0, tot = 0;
         CUDA_TRY(cudaMemGetInfo(&fr, &tot));
-        room = std::max(have, std::min(bytes, fr / 8));
+        room = std::max(have, std::min(kStaging, fr / 8));
     }
-    const int n = (int)std::min<size_t>(room / (fstride * sizeof(float)), (size_t)std::max(nsnap, 1));
-    const int few = std::max(4, (region_min_steps(g) + ks - 1) / ks);
-    if (n < std::min(few, std::max(nsnap, 1))) return PSDM_OK;
-    TRY(e->get(("reg_staging" + tag).c_str(), fstride * (size_t)n, stage));
+    int n = most;
+    if (bytes(most) > room) {
+        size_t one = 0;
+        for (const Staged& s : shots) one += s.g.field_cells() * sizeof(float);
+        n = (int)std::min<size_t>(room / one, (size_t)most);
+    }
+    for (const Staged& s : shots) {
+        const int few = std::max(4, (region_min_steps(s.g) + s.ks - 1) / s.ks);
+        if (n < std::min(few, std::max(s.nsnap, 1))) return PSDM_OK;
+    }
+    float* at = nullptr;
+    TRY(e->get("reg_staging", bytes(n) / sizeof(float), &at));
+    for (Staged& s : shots) {
+        s.stage = at;
+        at += s.g.field_cells() * (size_t)std::min(n, std::max(s.nsnap, 1));
+    }
     *nstage = n;
     return PSDM_OK;
 }
@@ -1775,7 +1801,7 @@ void mixed_backward_vars(const MixedBufs& mb, int nt, const float* h_w, RegSpec*
 // Forward passes of the mixed form: launches of up to nstage snapshots each,
 // every one followed by the conversion of what it staged.
 int region_mixed_forward(psdm_engine* e, RegPass& P, const std::vector<const MixedBufs*>& mb,
-                         const std::vector<float*>& stage, int nstage) {
+                         const std::vector<Staged>& staged, int nstage) {
     const size_t n = P.specs->size();
     std::vector<std::pair<int, int>> range(n, {0, 0});
     for (int c = 0;; ++c) {
@@ -1791,7 +1817,8 @@ int region_mixed_forward(psdm_engine* e, RegPass& P, const std::vector<const Mix
         for (size_t k = 0; k < n; ++k) {
             const int m0 = std::min(c * nstage, mb[k]->nsnap), cnt = std::min((c + 1) * nstage, mb[k]->nsnap) - m0;
             if (cnt <= 0) continue;
-            const int rc = launch_quantize_many(stage[k], mb[k]->amax + m0, mb[k]->snap16 + (size_t)m0 * mb[k]->fstride,
+            const int rc = launch_quantize_many(staged[k].stage, mb[k]->amax + m0,
+                                                mb[k]->snap16 + (size_t)m0 * mb[k]->fstride,
                                                 mb[k]->iscale + m0, (int)mb[k]->fstride, mb[k]->kind, cnt, e->stream);
             if (rc) return fail(PSDM_ERR_CUDA, "snapshot conversion launch: %s", cudaGetErrorString((cudaError_t)rc));
             e->launches += 1;
@@ -2130,12 +2157,12 @@ int region_mixed_shot(psdm_engine* e, Shot& s, const MixedBufs& mb, int NumRec, 
     TRY(region_plan(e, s.g, s.fs, pass_regions(e, s.g, s.fs), 0, &fw[0].plan));
     if (!fw[0].plan) return 1;
     bw[0].plan = fw[0].plan;
-    float* stage = nullptr;
+    std::vector<Staged> staged = {{s.g, mb.ks, mb.nsnap}};
     int nstage = 0;
-    TRY(mixed_stage(e, s.g, mb.ks, mb.nsnap, (size_t)512 << 20, "", &stage, &nstage));
+    TRY(mixed_stage(e, staged, &nstage));
     if (nstage == 0) return 1;
     TRY(forward_spec(s, nt_prop2, store_snap, d_S, w.zs, w.xs, nullptr, 0, 0, nullptr, nullptr, &fw[0]));
-    mixed_forward_vars(mb, stage, nstage, fw[0].var);
+    mixed_forward_vars(mb, staged[0].stage, nstage, fw[0].var);
     TRY(backward_spec(s, nt_taper, store_snap, nt_taper, d_tgt, 1, NumRec, w.zr.data(), w.xr.data(), nullptr, 1, 0,
                       nullptr, d_imgp, &bw[0]));
     mixed_backward_vars(mb, nt_taper, wts, &bw[0]);
@@ -2143,7 +2170,7 @@ int region_mixed_shot(psdm_engine* e, Shot& s, const MixedBufs& mb, int NumRec, 
     int rc = region_prepare(e, fw, "0", &F);
     if (rc == PSDM_OK) rc = region_prepare(e, bw, "1", &B);
     if (rc != PSDM_OK) return rc;
-    TRY(region_mixed_forward(e, F, {&mb}, {stage}, nstage));
+    TRY(region_mixed_forward(e, F, {&mb}, staged, nstage));
     e->fwd_steps += nt_prop2 - 1;
     TRY(e->record(1));
     CUDA_TRY(cudaMemsetAsync(d_imgp, 0, mb.fstride * sizeof(float), e->stream));
@@ -2692,9 +2719,9 @@ int batch_group_run(psdm_engine* e, const BatchJob& j, std::vector<BatchSlot>& s
     static_assert(psdm_engine::kRegPlans >= kMaxSlots, "a group holds a plan a shot");
     const std::vector<int> share = batch_shares(e, j, first, n);
     std::vector<RegSpec> fw(n), bw(n);
-    std::vector<float*> stage(n, nullptr);
+    std::vector<Staged> staged;
     std::vector<const MixedBufs*> mb(n);
-    int nstage = 1 << 30, pitch = 0;
+    int nstage = 0, pitch = 0;
     for (int k = 0; k < n; ++k) {
         BatchSlot& sl = slots[k];
         const psdm_shot& sh = j.shots[first + k];
@@ -2710,10 +2737,7 @@ int batch_group_run(psdm_engine* e, const BatchJob& j, std::vector<BatchSlot>& s
         float* d_F = nullptr;
         if (mixed) {
             TRY(mixed_bufs(e, sl.s, j.prm->precision, j.store_snap, sh.nt_prop2, sl.tag, &sl.mb));
-            int ns = 0;
-            TRY(mixed_stage(e, g, j.store_snap, nsnap, ((size_t)512 << 20) / n, sl.tag, &stage[k], &ns));
-            if (ns == 0) return 1;
-            nstage = std::min(nstage, ns);
+            staged.push_back({g, j.store_snap, nsnap});
         } else if (nsnap > 0) {
             TRY(e->get(("fields" + sl.tag).c_str(), fstride * nsnap, &d_F));
         }
@@ -2729,14 +2753,17 @@ int batch_group_run(psdm_engine* e, const BatchJob& j, std::vector<BatchSlot>& s
         mb[k] = &sl.mb;
         if (j.host_io) CUDA_TRY(cudaEventRecord(sl.staged, e->stream));
     }
-    if (mixed)
-        for (int k = 0; k < n; ++k) mixed_forward_vars(*mb[k], stage[k], nstage, fw[k].var);
+    if (mixed) {
+        TRY(mixed_stage(e, staged, &nstage));
+        if (nstage == 0) return 1;
+        for (int k = 0; k < n; ++k) mixed_forward_vars(*mb[k], staged[k].stage, nstage, fw[k].var);
+    }
     RegPass F, B;
     int rc = region_prepare(e, fw, "0", &F);
     if (rc == PSDM_OK) rc = region_prepare(e, bw, "1", &B);
     if (rc != PSDM_OK) return rc;
     if (mixed)
-        TRY(region_mixed_forward(e, F, mb, stage, nstage));
+        TRY(region_mixed_forward(e, F, mb, staged, nstage));
     else
         TRY(region_launch_all(e, 0, F));
     for (int k = 0; k < n; ++k) TRY(reset_state(e, &slots[k].s));  // second propagator call: fresh wavefield

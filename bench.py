@@ -79,6 +79,13 @@ def algorithmic_bytes(ny, nx_w, dpml, fs=1):
     return base + 4 * g["n_int"], base + 12 * g["n_int"], g
 
 
+def step_operations(g, which):
+    """FP32 adds and multiplies of one step: 29 a cell, 27 more a C-PML cell and
+    direction, 3 for a snapshot (forward) or 4 for an imaging update (backward)
+    of an interior cell."""
+    return 29 * g["n_act"] + 27 * (g["n_xpml"] + g["n_zpml"]) + (3 if which == "fwd" else 4) * g["n_int"]
+
+
 def algorithmic_bytes_mixed(ny, nx_w, dpml, fs, ks):
     """Compulsory bytes of one step of the mixed-precision form: the FP32
     propagation's 16 B per updated cell and C-PML bytes, and per interior
@@ -744,10 +751,13 @@ def run_gpu(args):
     bwd_us = st["bwd_ms"] * 1e3 / max(st["bwd_steps"], 1)
     dom = "bwd" if st["bwd_ms"] >= st["fwd_ms"] else "fwd"
     peak, peak_kind = _peaks()
-    # the region form keeps the wavefield, c2 and the image on the chip: a step moves its snapshot
+    # the region form keeps the wavefield, c2 and the image on the chip: a step is operations (adds and
+    # multiplies that may not be contracted), against the FP32 lanes' rate; in HBM it moves its snapshot
     us_dom = bwd_us if dom == "bwd" else fwd_us
-    achieved = 4 * g["n_int"] / (us_dom * 1e-6) / 1e9
-    one_step = (bwd_b if dom == "bwd" else fwd_b) / (us_dom * 1e-6) / 1e9
+    achieved = step_operations(g, dom) / (us_dom * 1e-6) / 1e12
+    mhz = clk.summary().get("sm_max_mhz") or 1965.0
+    peak_ops = torch.cuda.get_device_properties(dev).multi_processor_count * 128 * mhz * 1e6 / 1e12
+    hbm = 4 * g["n_int"] / (us_dom * 1e-6) / 1e9
     traffic = profiled_traffic(dom, "region_kernel_config2_ncu.md", "traffic_bytes_per_step")
 
     # end-to-end through the C ABI with pinned host buffers
@@ -822,9 +832,10 @@ def run_gpu(args):
                 "gcell_upd_per_s": gcell,
                 "kernel": {"fwd_us_per_step": fwd_us, "bwd_us_per_step": bwd_us, "fwd_bytes": fwd_b,
                            "bwd_bytes": bwd_b},
-                "roofline": {"bound": "shared memory and issue", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                             "frac": achieved / peak, "one_step_form_gbs": one_step, "traffic": traffic, "kernel": f"region_kernel<{dom}>, per time step",
-                             "peak_kind": peak_kind},
+                "roofline": {"bound": "shared memory and issue", "achieved": achieved, "peak": peak_ops,
+                             "unit": "TFLOP/s", "frac": achieved / peak_ops, "peak_kind": "nominal",
+                             "hbm_gbs": hbm, "hbm_frac": hbm / peak, "hbm_peak_kind": peak_kind, "traffic": traffic,
+                             "kernel": f"region_kernel<{dom}>, per time step"},
                 "gpu_launches": int(st["launches"]),
                 "clocks": clk.summary(),
                 "e2e": e2e,

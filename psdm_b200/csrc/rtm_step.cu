@@ -859,8 +859,9 @@ __global__ void __launch_bounds__(NT, 5) batch_step_kernel(const BatchParams bp)
             return;
         }
         // every other launch takes the list backwards: it begins with what the last one left in L2, and
-        // boundary tiles overlap interior ones (FP16 shots of 3000 x 2620: 3 in flight 1.09 -> 1.15 shots/s,
-        // 8 with checkpoints 0.859 -> 0.879)
+        // boundary tiles overlap interior ones (FP16 shots of 3000 x 2620, ten calls each: 8 in flight with
+        // checkpoints 0.866 -> 0.888 shots/s; 3 with every snapshot 1.09 -> 1.15 in the fastest calls, others
+        // of both down to 0.62 where the call gives its buffers back and takes them again)
         if (bp.counter_sel) b = total - 1 - b;
         int s = 0;
         while (s + 1 < bp.nslots && b >= bp.first[s + 1]) ++s;
